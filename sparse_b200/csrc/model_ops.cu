@@ -74,50 +74,141 @@ add_rmsnorm_kernel(__nv_bfloat16 *__restrict__ residual, const __nv_bfloat16 *__
       out[base + i] = __float2bfloat16_rn(__bfloat162float(weight[i]) * round_bf16(row[i] * inv));
 }
 
-// One CTA per token.  Rotates the first `rope_dim` elements of every q and k
-// head (pairs (i, i + rope_dim/2), angle pos * theta^(-2i/rope_dim)), writes q
-// back in place and k, v into the cache row of (sequence, position).
-__global__ void __launch_bounds__(128)
-rope_append_kernel(__nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restrict__ k,
-                   const __nv_bfloat16 *__restrict__ v, const int32_t *__restrict__ seq_of_token,
-                   const int32_t *__restrict__ pos_of_token, int n_q, int n_kv, int dk, int dv, int rope_dim,
-                   float theta, int s_max, __nv_bfloat16 *__restrict__ cache_k, __nv_bfloat16 *__restrict__ cache_v,
-                   int q_stride, int k_stride, int v_stride) {
+// Rotates the first `rope_dim` elements of every q and k head (pairs
+// (i, i + rope_dim/2), angle pos * theta^(-2i/rope_dim)), writes q back in place
+// and k, v into the cache row of (sequence, position).
+//
+// A token's angles are the same for every head: the CTA works out its
+// rope_dim/2 sines and cosines once, in shared memory, and the heads then move
+// as W-element vectors (W = 8: 16 bytes), all of a thread's loads independent.
+// HBM-bound at prefill (q, k, v read and written once); at a decode step's few
+// tokens it is the length of the chain position -> angle -> rows, so the token's
+// vectors are spread over `gridDim.y` CTAs.  (One sincosf per rotated element and
+// 2-byte accesses: 18 us at 8 tokens, 91 us at 4096 tokens of 16 heads of 128.)
+// W = 1 serves head widths, strides and addresses that are no whole vectors.
+constexpr int kRopeThreads = 256;
+constexpr int kRopeTable = 1024;      // angles kept in shared memory; wider heads compute them per element
+
+struct RopeSource {                   // element (token t, head h, i) at base + t*token + h*head + i
+  const __nv_bfloat16 *base;
+  int token, head;
+  __device__ __forceinline__ const __nv_bfloat16 *at(int t, int h) const {
+    return base + (size_t)t * token + (size_t)h * head;
+  }
+};
+
+__device__ __forceinline__ float2 rope_cos_sin(int pos, int j, float log_theta, int rope_dim) {
+  const float ang = (float)pos * __expf(-log_theta * (2.0f * (float)j / (float)rope_dim));
+  float sn, cs;
+  sincosf(ang, &sn, &cs);
+  return make_float2(round_bf16(cs), round_bf16(sn));
+}
+
+template <int W> struct RopeVec { uint32_t w[W / 2]; };
+template <> struct RopeVec<1> { unsigned short w; };
+
+template <int W>
+__device__ __forceinline__ RopeVec<W> rope_load(const __nv_bfloat16 *p) {
+  RopeVec<W> r;
+  if constexpr (W == 8) {
+    const uint4 q = *reinterpret_cast<const uint4 *>(p);
+    r.w[0] = q.x; r.w[1] = q.y; r.w[2] = q.z; r.w[3] = q.w;
+  } else {
+    r.w = *reinterpret_cast<const unsigned short *>(p);
+  }
+  return r;
+}
+template <int W>
+__device__ __forceinline__ void rope_store(__nv_bfloat16 *p, const RopeVec<W> &r) {
+  if constexpr (W == 8) *reinterpret_cast<uint4 *>(p) = make_uint4(r.w[0], r.w[1], r.w[2], r.w[3]);
+  else *reinterpret_cast<unsigned short *>(p) = r.w;
+}
+__device__ __forceinline__ float2 rope_pair(float a, float b, float2 cs) {
+  return make_float2(round_bf16(a * cs.x) + round_bf16(-b * cs.y), round_bf16(b * cs.x) + round_bf16(a * cs.y));
+}
+
+// src (lo half at src, hi half at src + half) rotated into dst, W pairs from pair j on
+template <int W>
+__device__ __forceinline__ void rope_rotate(const __nv_bfloat16 *src, __nv_bfloat16 *dst, int j, int half, int pos,
+                                            float log_theta, int rope_dim, const float2 *table) {
+  const RopeVec<W> lo = rope_load<W>(src + j), hi = rope_load<W>(src + j + half);
+  RopeVec<W> rl, rh;
+  if constexpr (W == 8) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 e = rope_pair(bf16_lo(lo.w[i]), bf16_lo(hi.w[i]), table[j + 2 * i]);
+      const float2 o = rope_pair(bf16_hi(lo.w[i]), bf16_hi(hi.w[i]), table[j + 2 * i + 1]);
+      rl.w[i] = pack_bf16x2(e.x, o.x);
+      rh.w[i] = pack_bf16x2(e.y, o.y);
+    }
+  } else {
+    const float2 cs = half <= kRopeTable ? table[j] : rope_cos_sin(pos, j, log_theta, rope_dim);
+    const float2 e = rope_pair(__bfloat162float(__ushort_as_bfloat16(lo.w)),
+                               __bfloat162float(__ushort_as_bfloat16(hi.w)), cs);
+    rl.w = __bfloat16_as_ushort(__float2bfloat16_rn(e.x));
+    rh.w = __bfloat16_as_ushort(__float2bfloat16_rn(e.y));
+  }
+  rope_store<W>(dst + j, rl);
+  rope_store<W>(dst + j + half, rh);
+}
+
+template <int W>
+__global__ void __launch_bounds__(kRopeThreads)
+rope_append_kernel(__nv_bfloat16 *__restrict__ q, int q_stride, RopeSource k_rot, RopeSource k_rest, RopeSource v,
+                   const int32_t *__restrict__ seq_of_token, const int32_t *__restrict__ pos_of_token, int n_q,
+                   int n_kv, int dk, int dv, int rope_dim, float theta, int s_max,
+                   __nv_bfloat16 *__restrict__ cache_k, __nv_bfloat16 *__restrict__ cache_v) {
+  __shared__ float2 table[kRopeTable];
+  pdl_launch_dependents();
+  pdl_wait();
   const int t = blockIdx.x;
   const int pos = pos_of_token[t], seq = seq_of_token[t];
   const int half = rope_dim >> 1;
   const float log_theta = __logf(theta);
-  // q heads, in place
-  for (int i = threadIdx.x; i < n_q * half; i += blockDim.x) {
-    const int h = i / half, j = i - h * half;
-    const float ang = (float)pos * __expf(-log_theta * (2.0f * (float)j / (float)rope_dim));
-    float sn, cs;
-    sincosf(ang, &sn, &cs);
-    sn = round_bf16(sn); cs = round_bf16(cs);
-    __nv_bfloat16 *p = q + (size_t)t * q_stride + (size_t)h * dk;
-    const float a = __bfloat162float(p[j]), b = __bfloat162float(p[j + half]);
-    p[j] = __float2bfloat16_rn(round_bf16(a * cs) + round_bf16(-b * sn));
-    p[j + half] = __float2bfloat16_rn(round_bf16(b * cs) + round_bf16(a * sn));
-  }
-  if (pos < 0 || pos >= s_max) return;
+  if (half <= kRopeTable)
+    for (int j = threadIdx.x; j < half; j += kRopeThreads) table[j] = rope_cos_sin(pos, j, log_theta, rope_dim);
+  __syncthreads();
+  const bool cached = pos >= 0 && pos < s_max;
   __nv_bfloat16 *ck = cache_k + ((size_t)seq * s_max + pos) * n_kv * dk;
   __nv_bfloat16 *cv = cache_v + ((size_t)seq * s_max + pos) * n_kv * dv;
-  for (int i = threadIdx.x; i < n_kv * dk; i += blockDim.x) {
-    const int h = i / dk, j = i - h * dk;
-    const __nv_bfloat16 *p = k + (size_t)t * k_stride + (size_t)h * dk;
-    float val = __bfloat162float(p[j]);
-    if (j < rope_dim) {
-      const int jj = j < half ? j : j - half;
-      const float ang = (float)pos * __expf(-log_theta * (2.0f * (float)jj / (float)rope_dim));
-      float sn, cs;
-      sincosf(ang, &sn, &cs);
-      sn = round_bf16(sn); cs = round_bf16(cs);
-      const float other = __bfloat162float(j < half ? p[j + half] : p[j - half]);
-      val = round_bf16(val * cs) + round_bf16((j < half ? -other : other) * sn);
+  // the token's vectors in one line: rotated q, rotated k, rest of k, v
+  const int per_rot = half / W, per_rest = (dk - rope_dim) / W, per_v = dv / W;
+  const int end_q = n_q * per_rot, end_k = end_q + n_kv * per_rot, end_rest = end_k + n_kv * per_rest;
+  const int end = cached ? end_rest + n_kv * per_v : end_q;
+  for (int i = blockIdx.y * kRopeThreads + threadIdx.x; i < end; i += gridDim.y * kRopeThreads) {
+    if (i < end_q) {
+      const int h = i / per_rot, j = (i - h * per_rot) * W;
+      __nv_bfloat16 *p = q + (size_t)t * q_stride + (size_t)h * dk;
+      rope_rotate<W>(p, p, j, half, pos, log_theta, rope_dim, table);
+    } else if (i < end_k) {
+      const int n = i - end_q, h = n / per_rot, j = (n - h * per_rot) * W;
+      rope_rotate<W>(k_rot.at(t, h), ck + (size_t)h * dk, j, half, pos, log_theta, rope_dim, table);
+    } else if (i < end_rest) {
+      const int n = i - end_k, h = n / per_rest, j = (n - h * per_rest) * W;
+      rope_store<W>(ck + (size_t)h * dk + rope_dim + j, rope_load<W>(k_rest.at(t, h) + j));
+    } else {
+      const int n = i - end_rest, h = n / per_v, j = (n - h * per_v) * W;
+      rope_store<W>(cv + (size_t)h * dv + j, rope_load<W>(v.at(t, h) + j));
     }
-    ck[i] = __float2bfloat16_rn(val);
   }
-  for (int i = threadIdx.x; i < n_kv * dv; i += blockDim.x) cv[i] = v[(size_t)t * v_stride + i];
+}
+
+int32_t launch_rope(__nv_bfloat16 *q, int q_stride, RopeSource k_rot, RopeSource k_rest, RopeSource v,
+                    const int32_t *seq_of_token, const int32_t *pos_of_token, int T, int n_q, int n_kv, int dk, int dv,
+                    int rope_dim, float theta, int s_max, void *cache_k, void *cache_v, cudaStream_t stream) {
+  const auto whole = [](const RopeSource &s) { return aligned(s.base, 16) && s.token % 8 == 0 && s.head % 8 == 0; };
+  const bool vec = dk % 8 == 0 && dv % 8 == 0 && rope_dim % 16 == 0 && rope_dim <= 2 * kRopeTable && q_stride % 8 == 0 &&
+                   aligned(q, 16) && whole(k_rot) && whole(k_rest) && whole(v) && aligned(cache_k, 16) && aligned(cache_v, 16);
+  // at most two waves' worth of CTAs: more would only repeat the angle table
+  const int items = (n_q * (rope_dim / 2) + n_kv * (dk - rope_dim / 2 + dv)) / (vec ? 8 : 1);
+  const int wanted = (items + kRopeThreads - 1) / kRopeThreads, room = (2 * 148 + T - 1) / T;
+  const dim3 grid(T, wanted < 1 ? 1 : wanted < room ? wanted : room);
+  auto kern = vec ? rope_append_kernel<8> : rope_append_kernel<1>;
+  SB_CUDA_CHECK(launch_pdl(kern, grid, dim3(kRopeThreads), 0, stream, q, q_stride, k_rot, k_rest, v, seq_of_token,
+                           pos_of_token, n_q, n_kv, dk, dv, rope_dim, theta, s_max,
+                           static_cast<__nv_bfloat16 *>(cache_k), static_cast<__nv_bfloat16 *>(cache_v)));
+  SB_LAUNCH_CHECK();
+  return SB_OK;
 }
 
 // Decode attention, split over the keys.  grid = (sequences * query heads,
@@ -263,12 +354,11 @@ int32_t sb_rope_append(void *q, const void *k, const void *v, const int32_t *seq
   if (T == 0) return SB_OK;
   if (!q || !k || !v || !seq_of_token || !pos_of_token || !cache_k || !cache_v)
     return fail(SB_E_INVALID_ARG, "sb_rope_append: null pointer");
-  rope_append_kernel<<<T, 128, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<__nv_bfloat16 *>(q), static_cast<const __nv_bfloat16 *>(k), static_cast<const __nv_bfloat16 *>(v),
-      seq_of_token, pos_of_token, n_q, n_kv, dk, dv, rope_dim, theta, s_max,
-      static_cast<__nv_bfloat16 *>(cache_k), static_cast<__nv_bfloat16 *>(cache_v), q_stride, k_stride, v_stride);
-  SB_LAUNCH_CHECK();
-  return SB_OK;
+  const __nv_bfloat16 *kk = static_cast<const __nv_bfloat16 *>(k);
+  return launch_rope(static_cast<__nv_bfloat16 *>(q), q_stride, RopeSource{kk, k_stride, dk},
+                     RopeSource{kk + rope_dim, k_stride, dk}, RopeSource{static_cast<const __nv_bfloat16 *>(v), v_stride, dv},
+                     seq_of_token, pos_of_token, T, n_q, n_kv, dk, dv, rope_dim, theta, s_max, cache_k, cache_v,
+                     static_cast<cudaStream_t>(stream));
 }
 
 size_t sb_attn_decode_workspace_bytes(int32_t B, int32_t n_q, int32_t dv, int32_t n_split) {
