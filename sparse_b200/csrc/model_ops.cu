@@ -44,6 +44,87 @@ __device__ __forceinline__ void load_bf16(const __nv_bfloat16 *p, float (&out)[E
 
 // One CTA per row.  h = bf16(residual + delta) (or residual alone); the row is
 // written back to `residual` when a delta was added; out = weight * bf16(h * rsqrt(mean(h^2) + eps)).
+//
+// HBM-bound at prefill: a row is read once as 16-byte vectors, stays in registers
+// (NV vectors a thread; a bf16 copy in shared memory for the sum of squares) and is
+// written once, residual and normalised.
+// (2-byte accesses and a row in shared memory: 17 us for 4096 rows of 2048, whose
+// bytes take 10 us.)  At a decode step's few rows it is one load round trip.
+template <int NV>
+__global__ void __launch_bounds__(kNormThreads)
+add_rmsnorm_vec_kernel(__nv_bfloat16 *__restrict__ residual, const __nv_bfloat16 *__restrict__ delta,
+                       const __nv_bfloat16 *__restrict__ delta2, const __nv_bfloat16 *__restrict__ weight, float eps,
+                       int H, __nv_bfloat16 *__restrict__ out) {
+  __shared__ float part[kNormThreads / 32];
+  __shared__ uint4 row[NV * kNormThreads];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int vecs = H >> 3;
+  const size_t base = (size_t)blockIdx.x * vecs;
+  uint4 *res = reinterpret_cast<uint4 *>(residual) + base;
+  const uint4 *d1 = reinterpret_cast<const uint4 *>(delta) + base, *d2 = reinterpret_cast<const uint4 *>(delta2) + base;
+  uint4 r[NV], a[NV], b[NV], w[NV];
+#pragma unroll
+  for (int n = 0; n < NV; ++n) {
+    const int i = threadIdx.x + n * kNormThreads;
+    r[n] = a[n] = b[n] = w[n] = make_uint4(0, 0, 0, 0);
+    if (i < vecs) {
+      r[n] = res[i];
+      if (delta != nullptr) a[n] = __ldg(d1 + i);
+      if (delta2 != nullptr) b[n] = __ldg(d2 + i);
+      if (out != nullptr) w[n] = __ldg(reinterpret_cast<const uint4 *>(weight) + i);
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < NV; ++n) {
+    const int i = threadIdx.x + n * kNormThreads;
+    uint32_t *rv = reinterpret_cast<uint32_t *>(&r[n]);
+    const uint32_t *av = reinterpret_cast<const uint32_t *>(&a[n]), *bv = reinterpret_cast<const uint32_t *>(&b[n]);
+    if (delta != nullptr) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        float lo = round_bf16(bf16_lo(rv[k]) + bf16_lo(av[k])), hi = round_bf16(bf16_hi(rv[k]) + bf16_hi(av[k]));
+        if (delta2 != nullptr) {
+          lo = round_bf16(lo + bf16_lo(bv[k]));
+          hi = round_bf16(hi + bf16_hi(bv[k]));
+        }
+        rv[k] = pack_bf16x2(lo, hi);
+      }
+      if (i < vecs) res[i] = r[n];
+    }
+    if (i < vecs) row[i] = r[n];
+  }
+  if (out == nullptr) return;
+  // The squares are summed in element order t, t + 256, ... per thread, as the
+  // kernel for ragged rows below does: the same bits whatever the row's alignment.
+  __syncthreads();
+  const __nv_bfloat16 *elem = reinterpret_cast<const __nv_bfloat16 *>(row);
+  float ss = 0.f;
+#pragma unroll 8
+  for (int i = threadIdx.x; i < H; i += kNormThreads) {
+    const float v = __bfloat162float(elem[i]);
+    ss += v * v;
+  }
+  ss = warp_sum(ss);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  float tot = 0.f;
+#pragma unroll
+  for (int i = 0; i < kNormThreads / 32; ++i) tot += part[i];
+  const float inv = rsqrtf(tot / (float)H + eps);
+#pragma unroll
+  for (int n = 0; n < NV; ++n) {
+    const int i = threadIdx.x + n * kNormThreads;
+    const uint32_t *rv = reinterpret_cast<const uint32_t *>(&r[n]), *wv = reinterpret_cast<const uint32_t *>(&w[n]);
+    uint32_t o[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      o[k] = pack_bf16x2(bf16_lo(wv[k]) * round_bf16(bf16_lo(rv[k]) * inv), bf16_hi(wv[k]) * round_bf16(bf16_hi(rv[k]) * inv));
+    if (i < vecs) reinterpret_cast<uint4 *>(out)[base + i] = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+}
+
+// The same for rows that are no whole 16-byte vectors (or not aligned to them).
 __global__ void __launch_bounds__(kNormThreads)
 add_rmsnorm_kernel(__nv_bfloat16 *__restrict__ residual, const __nv_bfloat16 *__restrict__ delta,
                    const __nv_bfloat16 *__restrict__ delta2, const __nv_bfloat16 *__restrict__ weight, float eps,
@@ -332,10 +413,18 @@ int32_t sb_add_rmsnorm(void *residual, const void *delta, const void *delta2, co
   if (T == 0) return SB_OK;
   if (!residual || (!out && !delta) || (out && !weight) || (delta2 && !delta))
     return fail(SB_E_INVALID_ARG, "sb_add_rmsnorm: null pointer");
-  add_rmsnorm_kernel<<<T, kNormThreads, (size_t)H * sizeof(float), static_cast<cudaStream_t>(stream)>>>(
-      static_cast<__nv_bfloat16 *>(residual), static_cast<const __nv_bfloat16 *>(delta),
-      static_cast<const __nv_bfloat16 *>(delta2), static_cast<const __nv_bfloat16 *>(weight), eps, H,
-      static_cast<__nv_bfloat16 *>(out));
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  __nv_bfloat16 *res = static_cast<__nv_bfloat16 *>(residual), *oo = static_cast<__nv_bfloat16 *>(out);
+  const __nv_bfloat16 *d1 = static_cast<const __nv_bfloat16 *>(delta), *d2 = static_cast<const __nv_bfloat16 *>(delta2);
+  const __nv_bfloat16 *ww = static_cast<const __nv_bfloat16 *>(weight);
+  if (H % 8 == 0 && aligned(res, 16) && aligned(d1, 16) && aligned(d2, 16) && aligned(ww, 16) && aligned(oo, 16)) {
+    const int nv = (H / 8 + kNormThreads - 1) / kNormThreads;
+    auto kern = nv == 1 ? add_rmsnorm_vec_kernel<1> : nv == 2 ? add_rmsnorm_vec_kernel<2>
+                        : nv <= 4 ? add_rmsnorm_vec_kernel<4> : add_rmsnorm_vec_kernel<8>;
+    SB_CUDA_CHECK(launch_pdl(kern, dim3(T), dim3(kNormThreads), 0, st, res, d1, d2, ww, eps, H, oo));
+  } else {
+    add_rmsnorm_kernel<<<T, kNormThreads, (size_t)H * sizeof(float), st>>>(res, d1, d2, ww, eps, H, oo);
+  }
   SB_LAUNCH_CHECK();
   return SB_OK;
 }

@@ -45,3 +45,25 @@ def test_rope_vectors_give_the_bits_of_single_elements(t, heads, dk, dv, rope_di
     for a, b in zip(*got):
         assert torch.equal(a, b)
     assert torch.equal(got[0][2][0, 1:t].reshape(t - 1, -1), v[1:])
+
+
+@pytest.mark.parametrize("t,h,with_delta", [(3, 8, True), (2, 504, True), (1, 2056, False), (2, 16384, True)])
+def test_rmsnorm_vectors_give_the_bits_of_single_elements(t, h, with_delta):
+    torch.manual_seed(h)
+    resid, delta = (torch.randn(t, h, device=DEV).to(BF) for _ in range(2))
+    w = torch.randn(h, device=DEV).to(BF)
+    got = []
+    for off in (0, 1):
+        if off and h > 12288:                         # (the element kernel's row must fit 48 KB as floats)
+            continue
+        r, d, o = _shifted(resid, off), _shifted(delta, off), _shifted(resid, off)
+        check(lib.sb_add_rmsnorm(r.data_ptr(), d.data_ptr() if with_delta else None, None, w.data_ptr(), 1e-6, t, h,
+                                 o.data_ptr(), _stream()), "sb_add_rmsnorm")
+        got.append((r, o))
+    torch.cuda.synchronize()
+    for r, o in got[1:]:
+        assert torch.equal(r, got[0][0]) and torch.equal(o, got[0][1])
+    x = (resid.float() + delta.float()).to(BF).float() if with_delta else resid.float()
+    want = w.float() * (x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + 1e-6)).to(BF).float()
+    # rsqrt and the fp32 mean may round differently: one bf16 step of the largest value
+    assert float((got[0][1].float() - want).abs().max()) <= 2.0 ** -7 * float(want.abs().max())
