@@ -31,17 +31,6 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
-template <int E>
-__device__ __forceinline__ void load_bf16(const __nv_bfloat16 *p, float (&out)[E]) {
-  static_assert(E % 2 == 0, "pairs");
-#pragma unroll
-  for (int e = 0; e < E; e += 2) {
-    const uint32_t w = *reinterpret_cast<const uint32_t *>(p + e);
-    out[e] = bf16_lo(w);
-    out[e + 1] = bf16_hi(w);
-  }
-}
-
 // One CTA per row.  h = bf16(residual + delta) (or residual alone); the row is
 // written back to `residual` when a delta was added; out = weight * bf16(h * rsqrt(mean(h^2) + eps)).
 //
@@ -293,111 +282,198 @@ int32_t launch_rope(__nv_bfloat16 *q, int q_stride, RopeSource k_rot, RopeSource
 }
 
 // Decode attention, split over the keys.  grid = (sequences * query heads,
-// splits); a CTA of 4 warps walks its slice of the cached keys, each warp every
-// fourth key, lanes owning DK/32 (DV/32) consecutive elements, online softmax
-// per warp; the warps and then the splits are merged by their running maxima.
-template <int DK, int DV>
-__global__ void __launch_bounds__(128)
+// splits).  HBM-bound: every cached key and value is read once, so what counts is
+// bytes in flight and instructions per byte.  Eight lanes share a key: lane i of
+// them owns the 16-byte vectors i, i + 8, ... of the key and of the value, so a
+// warp's load covers four keys in whole 128-byte lines, the score needs three
+// shuffles for four keys, and each of the 16 groups of a CTA keeps its own running
+// maximum; groups, then warps, then splits are merged by their maxima.
+// (One key per warp with 8-byte loads and five shuffles a key: 30 us for the
+// 137 MB of 8 sequences of 2049 positions with 16 heads of 128.)  Seven CTAs per
+// SM, where the head width lets the registers: the splits are cut for six.
+constexpr int kAttnThreads = 128;
+constexpr int kAttnLanes = 8;                                   // lanes per key
+constexpr int kAttnGroups = kAttnThreads / kAttnLanes;
+
+// 8 elements as fp32; A16: the address is a multiple of 16 bytes (else of 4)
+template <bool A16>
+__device__ __forceinline__ uint4 load_vec8(const __nv_bfloat16 *p) {
+  if (A16) return __ldg(reinterpret_cast<const uint4 *>(p));
+  const uint32_t *w = reinterpret_cast<const uint32_t *>(p);
+  return make_uint4(__ldg(w), __ldg(w + 1), __ldg(w + 2), __ldg(w + 3));
+}
+
+template <int DK, int DV, bool A16>
+__global__ void __launch_bounds__(kAttnThreads, DK <= 128 ? 7 : 5)
 attn_decode_kernel(const __nv_bfloat16 *__restrict__ q, int q_stride, const __nv_bfloat16 *__restrict__ cache_k,
                    const __nv_bfloat16 *__restrict__ cache_v, const int32_t *__restrict__ seq_lens, int n_q,
                    int n_kv, int s_max, float scale, int n_split, float *__restrict__ part) {
-  constexpr int EK = DK / 32, EV = DV / 32;
-  constexpr int U = 4;                        // keys a warp has in flight per iteration
+  constexpr int NK = DK / 64, NV = DV / 64;   // vectors a lane owns of a key / of a value
+  constexpr int U = 2;                        // keys a group has in flight per iteration
+  pdl_launch_dependents();
+  pdl_wait();
   const int bh = blockIdx.x, split = blockIdx.y;
   const int b = bh / n_q, h = bh - b * n_q;
   const int hk = h / (n_q / n_kv);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int group = threadIdx.x / kAttnLanes, li = threadIdx.x % kAttnLanes;
   const int len = min(seq_lens[b], s_max);
   const int per = (len + n_split - 1) / n_split;
   const int j0 = split * per, j1 = min(len, j0 + per);
-  float qv[EK];
+  float qv[NK * 8];
 #pragma unroll
-  for (int e = 0; e < EK; ++e)
-    qv[e] = __bfloat162float(q[(size_t)b * q_stride + (size_t)h * DK + lane * EK + e]) * scale;
-  float m = -INFINITY, l = 0.f, acc[EV];
+  for (int e = 0; e < NK * 8; ++e)
+    qv[e] = __bfloat162float(q[(size_t)b * q_stride + (size_t)h * DK + ((e >> 3) * kAttnLanes + li) * 8 + (e & 7)]) * scale;
+  float m = -INFINITY, l = 0.f, acc[NV * 8];
 #pragma unroll
-  for (int e = 0; e < EV; ++e) acc[e] = 0.f;
-  const __nv_bfloat16 *kb = cache_k + ((size_t)b * s_max * n_kv + hk) * DK + lane * EK;
-  const __nv_bfloat16 *vb = cache_v + ((size_t)b * s_max * n_kv + hk) * DV + lane * EV;
-  for (int j = j0 + warp * U; j < j1; j += 4 * U) {
-    float kv[U][EK], vv[U][EV], s[U];
+  for (int e = 0; e < NV * 8; ++e) acc[e] = 0.f;
+  const __nv_bfloat16 *kb = cache_k + ((size_t)b * s_max * n_kv + hk) * DK + li * 8;
+  const __nv_bfloat16 *vb = cache_v + ((size_t)b * s_max * n_kv + hk) * DV + li * 8;
+  for (int base = j0; base < j1; base += kAttnGroups * U) {
+    uint4 kv[U][NK], vv[U][NV];
+    float s[U];
+    bool ok[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int jj = min(j + u, j1 - 1);       // clamped: the duplicate is masked below
-      load_bf16<EK>(kb + (size_t)jj * n_kv * DK, kv[u]);
-      load_bf16<EV>(vb + (size_t)jj * n_kv * DV, vv[u]);
+      const int j = base + u * kAttnGroups + group;
+      ok[u] = j < j1;
+      const int jj = min(j, j1 - 1);          // clamped: a line its neighbours read too, masked below
+#pragma unroll
+      for (int n = 0; n < NK; ++n) kv[u][n] = load_vec8<A16>(kb + (size_t)jj * n_kv * DK + n * kAttnLanes * 8);
+#pragma unroll
+      for (int n = 0; n < NV; ++n) vv[u][n] = load_vec8<A16>(vb + (size_t)jj * n_kv * DV + n * kAttnLanes * 8);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      s[u] = 0.f;
+      float even = 0.f, odd = 0.f;
 #pragma unroll
-      for (int e = 0; e < EK; ++e) s[u] += qv[e] * kv[u][e];
+      for (int n = 0; n < NK; ++n) {
+        const uint32_t w[4] = {kv[u][n].x, kv[u][n].y, kv[u][n].z, kv[u][n].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          even += qv[n * 8 + 2 * i] * bf16_lo(w[i]);
+          odd += qv[n * 8 + 2 * i + 1] * bf16_hi(w[i]);
+        }
+      }
+      s[u] = even + odd;
     }
 #pragma unroll
-    for (int off = 16; off >= 1; off >>= 1)
+    for (int off = kAttnLanes / 2; off >= 1; off >>= 1)
 #pragma unroll
       for (int u = 0; u < U; ++u) s[u] += __shfl_xor_sync(0xffffffffu, s[u], off);
     float m_new = m;
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (j + u >= j1) s[u] = -INFINITY;
-      m_new = fmaxf(m_new, s[u]);
-    }
-    const float corr = __expf(m - m_new);
+    for (int u = 0; u < U; ++u)
+      if (ok[u]) m_new = fmaxf(m_new, s[u]);
+    // a group that has seen no key yet (or only scores of -inf) keeps its zero sums
+    const float corr = m == m_new ? 1.f : __expf(m - m_new);
     l *= corr;
 #pragma unroll
-    for (int e = 0; e < EV; ++e) acc[e] *= corr;
+    for (int e = 0; e < NV * 8; ++e) acc[e] *= corr;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const float p = __expf(s[u] - m_new);    // exp(-inf) = 0 for the masked keys
+      if (!ok[u]) continue;                   // a masked key adds nothing, whatever its clamped row holds
+      const float p = __expf(s[u] - m_new);
       l += p;
 #pragma unroll
-      for (int e = 0; e < EV; ++e) acc[e] += p * vv[u][e];
+      for (int n = 0; n < NV; ++n) {
+        const uint32_t w[4] = {vv[u][n].x, vv[u][n].y, vv[u][n].z, vv[u][n].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          acc[n * 8 + 2 * i] += p * bf16_lo(w[i]);
+          acc[n * 8 + 2 * i + 1] += p * bf16_hi(w[i]);
+        }
+      }
     }
     m = m_new;
   }
-  // merge the four warps
+  // merge the four groups of a warp, then the four warps
+#pragma unroll
+  for (int off = kAttnLanes; off <= 16; off <<= 1) {
+    const float mm = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+    const float c = m == -INFINITY ? 0.f : __expf(m - mm);      // (only scores of -inf: l is NaN, and NaN * 0 stays NaN)
+    l *= c;
+    l += __shfl_xor_sync(0xffffffffu, l, off);
+#pragma unroll
+    for (int e = 0; e < NV * 8; ++e) {
+      acc[e] *= c;
+      acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], off);
+    }
+    m = mm;
+  }
   __shared__ float sm[4], sl[4], sacc[4][DV];
   if (lane == 0) { sm[warp] = m; sl[warp] = l; }
+  if (lane < kAttnLanes) {
 #pragma unroll
-  for (int e = 0; e < EV; ++e) sacc[warp][lane * EV + e] = acc[e];
+    for (int e = 0; e < NV * 8; ++e) sacc[warp][((e >> 3) * kAttnLanes + li) * 8 + (e & 7)] = acc[e];
+  }
   __syncthreads();
-  if (warp == 0) {
-    float mm = fmaxf(fmaxf(sm[0], sm[1]), fmaxf(sm[2], sm[3]));
-    float ll = 0.f, out[EV];
+  float *dst = part + ((size_t)bh * n_split + split) * (DV + 2);
+  const float mm = fmaxf(fmaxf(sm[0], sm[1]), fmaxf(sm[2], sm[3]));
+  float c[4];
 #pragma unroll
-    for (int e = 0; e < EV; ++e) out[e] = 0.f;
-#pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      const float c = sm[w] == -INFINITY ? 0.f : __expf(sm[w] - mm);
-      ll += sl[w] * c;
-#pragma unroll
-      for (int e = 0; e < EV; ++e) out[e] += sacc[w][lane * EV + e] * c;
-    }
-    float *dst = part + ((size_t)bh * n_split + split) * (DV + 2);
-    if (lane == 0) { dst[0] = mm; dst[1] = ll; }
-#pragma unroll
-    for (int e = 0; e < EV; ++e) dst[2 + lane * EV + e] = out[e];
+  for (int w = 0; w < 4; ++w) c[w] = sm[w] == -INFINITY ? 0.f : __expf(sm[w] - mm);
+  if (threadIdx.x < DV)
+    dst[2 + threadIdx.x] = sacc[0][threadIdx.x] * c[0] + sacc[1][threadIdx.x] * c[1] + sacc[2][threadIdx.x] * c[2] +
+                           sacc[3][threadIdx.x] * c[3];
+  if (threadIdx.x == 0) {
+    dst[0] = mm;
+    dst[1] = sl[0] * c[0] + sl[1] * c[1] + sl[2] * c[2] + sl[3] * c[3];
   }
 }
 
+// One CTA of DV threads per (sequence, head).  The first warp turns the splits'
+// maxima into weights, so the sum over the splits is a run of independent loads
+// (with the weights worked out by every thread in the loop: 7.6 us at 56 splits).
+constexpr int kMaxSplit = 256;
 template <int DV>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(DV)
 attn_merge_kernel(const float *__restrict__ part, int n_split, __nv_bfloat16 *__restrict__ out) {
+  __shared__ float weight[kMaxSplit];
+  __shared__ float total;
+  pdl_launch_dependents();
+  pdl_wait();
   const int bh = blockIdx.x;
   const float *src = part + (size_t)bh * n_split * (DV + 2);
-  float mm = -INFINITY;
-  for (int s = 0; s < n_split; ++s) mm = fmaxf(mm, src[(size_t)s * (DV + 2)]);
-  for (int d = threadIdx.x; d < DV; d += blockDim.x) {
-    float ll = 0.f, acc = 0.f;
-    for (int s = 0; s < n_split; ++s) {
-      const float *p = src + (size_t)s * (DV + 2);
-      const float c = p[0] == -INFINITY ? 0.f : __expf(p[0] - mm);
-      ll += p[1] * c;
-      acc += p[2 + d] * c;
+  if (threadIdx.x < 32) {
+    float ms[kMaxSplit / 32], ls[kMaxSplit / 32], mm = -INFINITY, ll = 0.f;
+#pragma unroll
+    for (int i = 0; i < kMaxSplit / 32; ++i) {
+      const int s = threadIdx.x + 32 * i;
+      ms[i] = -INFINITY; ls[i] = 0.f;
+      if (s < n_split) { ms[i] = src[(size_t)s * (DV + 2)]; ls[i] = src[(size_t)s * (DV + 2) + 1]; }
+      mm = fmaxf(mm, ms[i]);
     }
-    out[(size_t)bh * DV + d] = __float2bfloat16_rn(ll > 0.f ? acc / ll : 0.f);
+    mm = warp_max(mm);
+#pragma unroll
+    for (int i = 0; i < kMaxSplit / 32; ++i) {
+      const float c = ms[i] == -INFINITY ? 0.f : __expf(ms[i] - mm);
+      ll += ls[i] * c;
+      if (threadIdx.x + 32 * i < n_split) weight[threadIdx.x + 32 * i] = c;
+    }
+    ll = warp_sum(ll);
+    if (threadIdx.x == 0) total = ll;
   }
+  __syncthreads();
+  float acc = 0.f;
+#pragma unroll 8
+  for (int s = 0; s < n_split; ++s) acc += src[(size_t)s * (DV + 2) + 2 + threadIdx.x] * weight[s];
+  out[(size_t)bh * DV + threadIdx.x] = __float2bfloat16_rn(total > 0.f ? acc / total : 0.f);
+}
+
+template <int DK, int DV>
+int32_t launch_attn_decode(const __nv_bfloat16 *q, int q_stride, const __nv_bfloat16 *cache_k,
+                           const __nv_bfloat16 *cache_v, const int32_t *seq_lens, int B, int n_q, int n_kv, int s_max,
+                           float scale, int n_split, float *part, __nv_bfloat16 *out, cudaStream_t stream) {
+  auto kern = aligned(cache_k, 16) && aligned(cache_v, 16) ? attn_decode_kernel<DK, DV, true>
+                                                           : attn_decode_kernel<DK, DV, false>;
+  SB_CUDA_CHECK(launch_pdl(kern, dim3(B * n_q, n_split), dim3(kAttnThreads), 0, stream, q, q_stride, cache_k, cache_v,
+                           seq_lens, n_q, n_kv, s_max, scale, n_split, part));
+  SB_LAUNCH_CHECK();
+  SB_CUDA_CHECK(launch_pdl(attn_merge_kernel<DV>, dim3(B * n_q), dim3(DV), 0, stream,
+                           static_cast<const float *>(part), n_split, out));
+  SB_LAUNCH_CHECK();
+  return SB_OK;
 }
 
 }  // namespace
@@ -468,29 +544,18 @@ int32_t sb_attn_decode(const void *q, int32_t q_stride, const void *cache_k, con
   if (ws_bytes < sb_attn_decode_workspace_bytes(B, n_q, dv, n_split))
     return fail(SB_E_WORKSPACE, "sb_attn_decode: workspace too small");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const dim3 grid(B * n_q, n_split);
   const __nv_bfloat16 *qq = static_cast<const __nv_bfloat16 *>(q);
   const __nv_bfloat16 *kk = static_cast<const __nv_bfloat16 *>(cache_k);
   const __nv_bfloat16 *vv = static_cast<const __nv_bfloat16 *>(cache_v);
   float *part = static_cast<float *>(ws);
   __nv_bfloat16 *oo = static_cast<__nv_bfloat16 *>(out);
-  if (dk == 128 && dv == 128) {
-    attn_decode_kernel<128, 128><<<grid, 128, 0, st>>>(qq, q_stride, kk, vv, seq_lens, n_q, n_kv, s_max, scale, n_split, part);
-    SB_LAUNCH_CHECK();
-    attn_merge_kernel<128><<<B * n_q, 128, 0, st>>>(part, n_split, oo);
-  } else if (dk == 192 && dv == 128) {
-    attn_decode_kernel<192, 128><<<grid, 128, 0, st>>>(qq, q_stride, kk, vv, seq_lens, n_q, n_kv, s_max, scale, n_split, part);
-    SB_LAUNCH_CHECK();
-    attn_merge_kernel<128><<<B * n_q, 128, 0, st>>>(part, n_split, oo);
-  } else if (dk == 64 && dv == 64) {
-    attn_decode_kernel<64, 64><<<grid, 128, 0, st>>>(qq, q_stride, kk, vv, seq_lens, n_q, n_kv, s_max, scale, n_split, part);
-    SB_LAUNCH_CHECK();
-    attn_merge_kernel<64><<<B * n_q, 128, 0, st>>>(part, n_split, oo);
-  } else {
-    return fail(SB_E_UNSUPPORTED, "sb_attn_decode: head dims (%d,%d) not built (128/128, 192/128, 64/64)", dk, dv);
-  }
-  SB_LAUNCH_CHECK();
-  return SB_OK;
+  if (dk == 128 && dv == 128)
+    return launch_attn_decode<128, 128>(qq, q_stride, kk, vv, seq_lens, B, n_q, n_kv, s_max, scale, n_split, part, oo, st);
+  if (dk == 192 && dv == 128)
+    return launch_attn_decode<192, 128>(qq, q_stride, kk, vv, seq_lens, B, n_q, n_kv, s_max, scale, n_split, part, oo, st);
+  if (dk == 64 && dv == 64)
+    return launch_attn_decode<64, 64>(qq, q_stride, kk, vv, seq_lens, B, n_q, n_kv, s_max, scale, n_split, part, oo, st);
+  return fail(SB_E_UNSUPPORTED, "sb_attn_decode: head dims (%d,%d) not built (128/128, 192/128, 64/64)", dk, dv);
 }
 
 }  // extern "C"

@@ -1,6 +1,8 @@
 """GPU: the decode-loop kernels at the edges of their vector paths, against the same
 call on tensors that take the other path (bits where the arithmetic is the same)
 or against plain PyTorch fp32."""
+import math
+
 import pytest
 import torch
 
@@ -67,3 +69,32 @@ def test_rmsnorm_vectors_give_the_bits_of_single_elements(t, h, with_delta):
     want = w.float() * (x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + 1e-6)).to(BF).float()
     # rsqrt and the fp32 mean may round differently: one bf16 step of the largest value
     assert float((got[0][1].float() - want).abs().max()) <= 2.0 ** -7 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("n_q,n_kv,dk,dv", [(4, 4, 128, 128), (2, 2, 192, 128), (4, 2, 64, 64)])
+@pytest.mark.parametrize("n_split,shift", [(1, 0), (3, 2), (256, 0)])
+def test_attn_decode_key_group_edges(n_q, n_kv, dk, dv, n_split, shift):
+    """Lengths around the 16 keys of a CTA's groups and its 32 per iteration, more splits
+    than keys, caches on 4-byte boundaries."""
+    torch.manual_seed(dk + n_split)
+    lens = [0, 1, 15, 16, 17, 31, 32, 33, 97]
+    b, s_max = len(lens), max(lens)
+    q = torch.randn(b, n_q, dk, device=DEV).to(BF)
+    ck = _shifted(torch.randn(b, s_max, n_kv, dk, device=DEV).to(BF), shift)
+    cv = _shifted(torch.randn(b, s_max, n_kv, dv, device=DEV).to(BF), shift)
+    cv[2, 15:] = float("inf")                         # past the length: read by nobody's sum
+    seq_lens = torch.tensor(lens, dtype=torch.int32, device=DEV)
+    ws = torch.empty(lib.sb_attn_decode_workspace_bytes(b, n_q, dv, n_split), dtype=torch.uint8, device=DEV)
+    out = torch.empty(b, n_q, dv, dtype=BF, device=DEV)
+    check(lib.sb_attn_decode(q.data_ptr(), 0, ck.data_ptr(), cv.data_ptr(), seq_lens.data_ptr(), b, n_q, n_kv, dk, dv,
+                             s_max, 1.0 / math.sqrt(dk), n_split, ws.data_ptr(), ws.numel(), out.data_ptr(), _stream()),
+          "sb_attn_decode")
+    torch.cuda.synchronize()
+    assert float(out[0].abs().max()) == 0.0
+    for i, n in enumerate(lens[1:], 1):
+        kk = ck[i, :n].float().repeat_interleave(n_q // n_kv, dim=1)
+        vv = cv[i, :n].float().repeat_interleave(n_q // n_kv, dim=1)
+        p = torch.softmax(torch.einsum("hd,nhd->hn", q[i].float(), kk) / math.sqrt(dk), dim=-1)
+        want = torch.einsum("hn,nhd->hd", p, vv)
+        # fp32 sums, one rounding to bf16: half a step of 2^-8 of a value, and __expf's 2^-21
+        assert float(((out[i].float() - want).abs() - 2.0 ** -8 * want.abs()).max()) < 1e-4
