@@ -574,6 +574,15 @@ int32_t sb_moe_layer_forward(const sb_moe_layer *layer, int32_t *status, void *s
  *                  k_stride, v_stride: elements between consecutive tokens
  *                  (0 = densely packed), so q, k, v may be column slices of
  *                  one fused projection output.
+ * sb_rmsnorm_rows  out [T,H] = weight * bf16(row * rsqrt(mean(row^2) + eps)) of rows
+ *                  that lie `row_stride` elements apart (column slices of a
+ *                  projection output); the rows themselves are not written.
+ * sb_rope_append_mla  sb_rope_append for heads whose rotated key part is shared:
+ *                  q [T,n_heads,rope_dim+nope_dim] rotated in place; k_pe
+ *                  [T,rope_dim] is rotated into every head of cache_k, the rest of
+ *                  a head's key and its value come from kv
+ *                  [T,n_heads,nope_dim+dv].  Same arithmetic, no assembled copy of
+ *                  k and v.
  * sb_attn_decode   one query per sequence, q [B,n_q,dk] (q_stride elements
  *                  between sequences, 0 = packed), against the first
  *                  seq_lens[b] (device int32) cached positions; softmax in fp32;
@@ -584,6 +593,12 @@ int32_t sb_moe_layer_forward(const sb_moe_layer *layer, int32_t *status, void *s
  */
 int32_t sb_add_rmsnorm(void *residual, const void *delta, const void *delta2, const void *weight, float eps,
                        int32_t T, int32_t H, void *out, void *stream);
+int32_t sb_rmsnorm_rows(const void *rows, int32_t row_stride, const void *weight, float eps, int32_t T, int32_t H,
+                        void *out, void *stream);
+int32_t sb_rope_append_mla(void *q, const void *k_pe, const void *kv, const int32_t *seq_of_token,
+                           const int32_t *pos_of_token, int32_t T, int32_t n_heads, int32_t rope_dim, int32_t nope_dim,
+                           int32_t dv, float theta, int32_t s_max, void *cache_k, void *cache_v, int32_t q_stride,
+                           int32_t k_pe_stride, int32_t kv_stride, void *stream);
 int32_t sb_rope_append(void *q, const void *k, const void *v, const int32_t *seq_of_token,
                        const int32_t *pos_of_token, int32_t T, int32_t n_q, int32_t n_kv, int32_t dk, int32_t dv,
                        int32_t rope_dim, float theta, int32_t s_max, void *cache_k, void *cache_v, int32_t q_stride,

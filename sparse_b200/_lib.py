@@ -93,6 +93,9 @@ SIGNATURES: Dict[str, Tuple[object, list]] = {
     "sb_add_rmsnorm": (i32, [vp, vp, vp, vp, C.c_float, i32, i32, vp, vp]),
     "sb_rope_append": (i32, [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, C.c_float, i32, vp, vp, i32, i32, i32,
                              vp]),
+    "sb_rmsnorm_rows": (i32, [vp, i32, vp, C.c_float, i32, i32, vp, vp]),
+    "sb_rope_append_mla": (i32, [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, C.c_float, i32, vp, vp, i32, i32, i32,
+                                 vp]),
     "sb_attn_decode_workspace_bytes": (sz, [i32, i32, i32, i32]),
     "sb_attn_decode": (i32, [vp, i32, vp, vp, vp, i32, i32, i32, i32, i32, i32, C.c_float, i32, vp, sz, vp, vp]),
     "sb_moe_layer_struct_bytes": (sz, []),

@@ -41,16 +41,16 @@ __device__ __forceinline__ float warp_max(float v) {
 // bytes take 10 us.)  At a decode step's few rows it is one load round trip.
 template <int NV>
 __global__ void __launch_bounds__(kNormThreads)
-add_rmsnorm_vec_kernel(__nv_bfloat16 *__restrict__ residual, const __nv_bfloat16 *__restrict__ delta,
-                       const __nv_bfloat16 *__restrict__ delta2, const __nv_bfloat16 *__restrict__ weight, float eps,
-                       int H, __nv_bfloat16 *__restrict__ out) {
+add_rmsnorm_vec_kernel(__nv_bfloat16 *__restrict__ residual, size_t res_stride,
+                       const __nv_bfloat16 *__restrict__ delta, const __nv_bfloat16 *__restrict__ delta2,
+                       const __nv_bfloat16 *__restrict__ weight, float eps, int H, __nv_bfloat16 *__restrict__ out) {
   __shared__ float part[kNormThreads / 32];
   __shared__ uint4 row[NV * kNormThreads];
   pdl_launch_dependents();
   pdl_wait();
   const int vecs = H >> 3;
   const size_t base = (size_t)blockIdx.x * vecs;
-  uint4 *res = reinterpret_cast<uint4 *>(residual) + base;
+  uint4 *res = reinterpret_cast<uint4 *>(residual + blockIdx.x * res_stride);
   const uint4 *d1 = reinterpret_cast<const uint4 *>(delta) + base, *d2 = reinterpret_cast<const uint4 *>(delta2) + base;
   uint4 r[NV], a[NV], b[NV], w[NV];
 #pragma unroll
@@ -115,19 +115,20 @@ add_rmsnorm_vec_kernel(__nv_bfloat16 *__restrict__ residual, const __nv_bfloat16
 
 // The same for rows that are no whole 16-byte vectors (or not aligned to them).
 __global__ void __launch_bounds__(kNormThreads)
-add_rmsnorm_kernel(__nv_bfloat16 *__restrict__ residual, const __nv_bfloat16 *__restrict__ delta,
+add_rmsnorm_kernel(__nv_bfloat16 *__restrict__ residual, size_t res_stride, const __nv_bfloat16 *__restrict__ delta,
                    const __nv_bfloat16 *__restrict__ delta2, const __nv_bfloat16 *__restrict__ weight, float eps,
                    int H, __nv_bfloat16 *__restrict__ out) {
   extern __shared__ float row[];                 // H floats
   __shared__ float part[kNormThreads / 32];
   const size_t base = (size_t)blockIdx.x * H;
+  residual += blockIdx.x * res_stride;
   float ss = 0.f;
   for (int i = threadIdx.x; i < H; i += kNormThreads) {
-    float v = __bfloat162float(residual[base + i]);
+    float v = __bfloat162float(residual[i]);
     if (delta != nullptr) {
       v = round_bf16(v + __bfloat162float(delta[base + i]));
       if (delta2 != nullptr) v = round_bf16(v + __bfloat162float(delta2[base + i]));
-      residual[base + i] = __float2bfloat16_rn(v);
+      residual[i] = __float2bfloat16_rn(v);
     }
     row[i] = v;
     ss += v * v;
@@ -142,6 +143,25 @@ add_rmsnorm_kernel(__nv_bfloat16 *__restrict__ residual, const __nv_bfloat16 *__
   if (out != nullptr)
     for (int i = threadIdx.x; i < H; i += kNormThreads)
       out[base + i] = __float2bfloat16_rn(__bfloat162float(weight[i]) * round_bf16(row[i] * inv));
+}
+
+int32_t launch_add_rmsnorm(void *residual, int res_stride, const void *delta, const void *delta2, const void *weight,
+                           float eps, int T, int H, void *out, cudaStream_t stream) {
+  __nv_bfloat16 *res = static_cast<__nv_bfloat16 *>(residual), *oo = static_cast<__nv_bfloat16 *>(out);
+  const __nv_bfloat16 *d1 = static_cast<const __nv_bfloat16 *>(delta), *d2 = static_cast<const __nv_bfloat16 *>(delta2);
+  const __nv_bfloat16 *ww = static_cast<const __nv_bfloat16 *>(weight);
+  if (H % 8 == 0 && res_stride % 8 == 0 && aligned(res, 16) && aligned(d1, 16) && aligned(d2, 16) && aligned(ww, 16) &&
+      aligned(oo, 16)) {
+    const int nv = (H / 8 + kNormThreads - 1) / kNormThreads;
+    auto kern = nv == 1 ? add_rmsnorm_vec_kernel<1> : nv == 2 ? add_rmsnorm_vec_kernel<2>
+                        : nv <= 4 ? add_rmsnorm_vec_kernel<4> : add_rmsnorm_vec_kernel<8>;
+    SB_CUDA_CHECK(launch_pdl(kern, dim3(T), dim3(kNormThreads), 0, stream, res, (size_t)res_stride, d1, d2, ww, eps, H, oo));
+  } else {
+    add_rmsnorm_kernel<<<T, kNormThreads, (size_t)H * sizeof(float), stream>>>(res, (size_t)res_stride, d1, d2, ww, eps,
+                                                                               H, oo);
+  }
+  SB_LAUNCH_CHECK();
+  return SB_OK;
 }
 
 // Rotates the first `rope_dim` elements of every q and k head (pairs
@@ -489,20 +509,18 @@ int32_t sb_add_rmsnorm(void *residual, const void *delta, const void *delta2, co
   if (T == 0) return SB_OK;
   if (!residual || (!out && !delta) || (out && !weight) || (delta2 && !delta))
     return fail(SB_E_INVALID_ARG, "sb_add_rmsnorm: null pointer");
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  __nv_bfloat16 *res = static_cast<__nv_bfloat16 *>(residual), *oo = static_cast<__nv_bfloat16 *>(out);
-  const __nv_bfloat16 *d1 = static_cast<const __nv_bfloat16 *>(delta), *d2 = static_cast<const __nv_bfloat16 *>(delta2);
-  const __nv_bfloat16 *ww = static_cast<const __nv_bfloat16 *>(weight);
-  if (H % 8 == 0 && aligned(res, 16) && aligned(d1, 16) && aligned(d2, 16) && aligned(ww, 16) && aligned(oo, 16)) {
-    const int nv = (H / 8 + kNormThreads - 1) / kNormThreads;
-    auto kern = nv == 1 ? add_rmsnorm_vec_kernel<1> : nv == 2 ? add_rmsnorm_vec_kernel<2>
-                        : nv <= 4 ? add_rmsnorm_vec_kernel<4> : add_rmsnorm_vec_kernel<8>;
-    SB_CUDA_CHECK(launch_pdl(kern, dim3(T), dim3(kNormThreads), 0, st, res, d1, d2, ww, eps, H, oo));
-  } else {
-    add_rmsnorm_kernel<<<T, kNormThreads, (size_t)H * sizeof(float), st>>>(res, d1, d2, ww, eps, H, oo);
-  }
-  SB_LAUNCH_CHECK();
-  return SB_OK;
+  return launch_add_rmsnorm(residual, H, delta, delta2, weight, eps, T, H, out, static_cast<cudaStream_t>(stream));
+}
+
+int32_t sb_rmsnorm_rows(const void *rows, int32_t row_stride, const void *weight, float eps, int32_t T, int32_t H,
+                        void *out, void *stream) {
+  if (T < 0 || H <= 0 || H > 16384 || row_stride < H)
+    return fail(SB_E_INVALID_ARG, "sb_rmsnorm_rows: bad shape (T=%d H=%d stride=%d)", T, H, row_stride);
+  if (T == 0) return SB_OK;
+  if (!rows || !weight || !out) return fail(SB_E_INVALID_ARG, "sb_rmsnorm_rows: null pointer");
+  // (without a delta the kernel does not write to its source rows)
+  return launch_add_rmsnorm(const_cast<void *>(rows), row_stride, nullptr, nullptr, weight, eps, T, H, out,
+                            static_cast<cudaStream_t>(stream));
 }
 
 int32_t sb_rope_append(void *q, const void *k, const void *v, const int32_t *seq_of_token,
@@ -523,6 +541,26 @@ int32_t sb_rope_append(void *q, const void *k, const void *v, const int32_t *seq
   return launch_rope(static_cast<__nv_bfloat16 *>(q), q_stride, RopeSource{kk, k_stride, dk},
                      RopeSource{kk + rope_dim, k_stride, dk}, RopeSource{static_cast<const __nv_bfloat16 *>(v), v_stride, dv},
                      seq_of_token, pos_of_token, T, n_q, n_kv, dk, dv, rope_dim, theta, s_max, cache_k, cache_v,
+                     static_cast<cudaStream_t>(stream));
+}
+
+int32_t sb_rope_append_mla(void *q, const void *k_pe, const void *kv, const int32_t *seq_of_token,
+                           const int32_t *pos_of_token, int32_t T, int32_t n_heads, int32_t rope_dim, int32_t nope_dim,
+                           int32_t dv, float theta, int32_t s_max, void *cache_k, void *cache_v, int32_t q_stride,
+                           int32_t k_pe_stride, int32_t kv_stride, void *stream) {
+  const int dk = rope_dim + nope_dim;
+  if (T < 0 || n_heads < 1 || rope_dim < 0 || (rope_dim & 1) || nope_dim < 0 || dk < 2 || dv < 1 || s_max < 1)
+    return fail(SB_E_INVALID_ARG, "sb_rope_append_mla: bad shape");
+  if (q_stride < n_heads * dk || k_pe_stride < rope_dim || kv_stride < n_heads * (nope_dim + dv))
+    return fail(SB_E_INVALID_ARG, "sb_rope_append_mla: a token stride is smaller than the token");
+  if (T == 0) return SB_OK;
+  if (!q || !k_pe || !kv || !seq_of_token || !pos_of_token || !cache_k || !cache_v)
+    return fail(SB_E_INVALID_ARG, "sb_rope_append_mla: null pointer");
+  const __nv_bfloat16 *rest = static_cast<const __nv_bfloat16 *>(kv);
+  return launch_rope(static_cast<__nv_bfloat16 *>(q), q_stride,
+                     RopeSource{static_cast<const __nv_bfloat16 *>(k_pe), k_pe_stride, 0},
+                     RopeSource{rest, kv_stride, nope_dim + dv}, RopeSource{rest + nope_dim, kv_stride, nope_dim + dv},
+                     seq_of_token, pos_of_token, T, n_heads, n_heads, dk, dv, rope_dim, theta, s_max, cache_k, cache_v,
                      static_cast<cudaStream_t>(stream));
 }
 

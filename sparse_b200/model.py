@@ -128,8 +128,10 @@ class ShapedMoeModel:
             ly.ln2 = torch.ones((h,), dtype=bf, device=device)
             if cfg.attention == "mla":
                 nope = dk - cfg.rope_dim
-                ly.wq = _normal((nh * dk, h), device, s0 + 1)
-                ly.wkv_a = _normal((cfg.kv_lora_rank + cfg.rope_dim, h), device, s0 + 2)
+                # one matrix: the query rows, then the latent and rotary key rows
+                ly.wq_kva = torch.cat([_normal((nh * dk, h), device, s0 + 1),
+                                       _normal((cfg.kv_lora_rank + cfg.rope_dim, h), device, s0 + 2)])
+                ly.wq, ly.wkv_a = ly.wq_kva[:nh * dk], ly.wq_kva[nh * dk:]
                 ly.kv_norm = torch.ones((cfg.kv_lora_rank,), dtype=bf, device=device)
                 ly.wkv_b = _normal((nh * (nope + dv), cfg.kv_lora_rank), device, s0 + 3)
                 ly.bqkv = None
@@ -176,31 +178,36 @@ class ShapedMoeModel:
                                  out.data_ptr(), self._s()), "sb_add_rmsnorm")
         return out
 
-    def _qkv(self, ly: _Layer, x: torch.Tensor):
+    def _qkv_rope_append(self, ly: _Layer, x: torch.Tensor, seq_of_token, pos_of_token) -> torch.Tensor:
+        """Projections of the rows, rotary embedding, keys and values into the cache;
+        returns the rotated queries (a column slice of the projection output)."""
         cfg = self.cfg
         nh, nkv, dk, dv, t = cfg.n_heads, cfg.n_kv_heads, cfg.qk_dim, cfg.v_dim, x.shape[0]
         if cfg.attention == "mla":
-            nope, rope = dk - cfg.rope_dim, cfg.rope_dim
-            q = F.linear(x, ly.wq)                                     # per head: [rope | nope]
-            kv_a = F.linear(x, ly.wkv_a)
-            c_kv = kv_a[:, :cfg.kv_lora_rank].contiguous()
-            k_pe = kv_a[:, cfg.kv_lora_rank:]
-            c_kv = self._norm(c_kv, None, ly.kv_norm)
-            kv = F.linear(c_kv, ly.wkv_b).view(t, nh, nope + dv)
-            k = torch.cat([k_pe.unsqueeze(1).expand(t, nh, rope), kv[:, :, :nope]], dim=2).reshape(t, nh * dk)
-            v = kv[:, :, nope:].reshape(t, nh * dv)
-            return q, k, v
+            nope, rope, lora = dk - cfg.rope_dim, cfg.rope_dim, cfg.kv_lora_rank
+            if t <= _lib.DECODE_MAX_TOKENS:      # a few rows: one launch over both weights
+                q_kva = F.linear(x, ly.wq_kva)                         # q per head: [rope | nope]
+                q, kv_a = q_kva[:, :nh * dk], q_kva[:, nh * dk:]
+            else:
+                q, kv_a = F.linear(x, ly.wq), F.linear(x, ly.wkv_a)
+            latent, k_pe = kv_a[:, :lora], kv_a[:, lora:]
+            c_kv = torch.empty((t, lora), dtype=x.dtype, device=x.device)
+            check(lib.sb_rmsnorm_rows(latent.data_ptr(), latent.stride(0), ly.kv_norm.data_ptr(), cfg.rms_eps, t, lora,
+                                      c_kv.data_ptr(), self._s()), "sb_rmsnorm_rows")
+            kv = F.linear(c_kv, ly.wkv_b)                              # per head: [nope | v]
+            check(lib.sb_rope_append_mla(q.data_ptr(), k_pe.data_ptr(), kv.data_ptr(), seq_of_token.data_ptr(),
+                                         pos_of_token.data_ptr(), t, nh, rope, nope, dv, cfg.rope_theta, self.max_seq,
+                                         ly.cache_k.data_ptr(), ly.cache_v.data_ptr(), q.stride(0), k_pe.stride(0),
+                                         kv.stride(0), self._s()), "sb_rope_append_mla")
+            return q
         # column slices of the fused projection: the kernels take the token stride
         qkv = F.linear(x, ly.wqkv, ly.bqkv)
-        return qkv[:, :nh * dk], qkv[:, nh * dk:nh * dk + nkv * dk], qkv[:, nh * dk + nkv * dk:]
-
-    def _rope_append(self, ly: _Layer, q, k, v, seq_of_token, pos_of_token) -> None:
-        cfg = self.cfg
+        q, k, v = qkv[:, :nh * dk], qkv[:, nh * dk:nh * dk + nkv * dk], qkv[:, nh * dk + nkv * dk:]
         check(lib.sb_rope_append(q.data_ptr(), k.data_ptr(), v.data_ptr(), seq_of_token.data_ptr(),
-                                 pos_of_token.data_ptr(), q.shape[0], cfg.n_heads, cfg.n_kv_heads, cfg.qk_dim,
-                                 cfg.v_dim, cfg.rope_dim, cfg.rope_theta, self.max_seq, ly.cache_k.data_ptr(),
-                                 ly.cache_v.data_ptr(), q.stride(0), k.stride(0), v.stride(0), self._s()),
-              "sb_rope_append")
+                                 pos_of_token.data_ptr(), t, nh, nkv, dk, dv, cfg.rope_dim, cfg.rope_theta,
+                                 self.max_seq, ly.cache_k.data_ptr(), ly.cache_v.data_ptr(), q.stride(0), k.stride(0),
+                                 v.stride(0), self._s()), "sb_rope_append")
+        return q
 
     # When set to a list, every MoE call appends (layer index, input rows, chosen experts):
     # what `rs_train.collect_pairs` turns into predictor training data.
@@ -234,8 +241,7 @@ class ShapedMoeModel:
         delta = None
         for ly in self.layers:
             x = self._norm(resid, delta, ly.ln1)
-            q, k, v = self._qkv(ly, x)
-            self._rope_append(ly, q, k, v, seq, pos)
+            q = self._qkv_rope_append(ly, x, seq, pos)
             qh = q.reshape(b, tc, nh, dk).transpose(1, 2)
             kh = ly.cache_k[:b, :kv_len].transpose(1, 2)
             vh = ly.cache_v[:b, :kv_len].transpose(1, 2)
@@ -280,8 +286,7 @@ class ShapedMoeModel:
         delta = None
         for ly in self.layers:
             x = self._norm(resid, delta, ly.ln1)
-            q, k, v = self._qkv(ly, x)
-            self._rope_append(ly, q, k, v, self.seq_ids, self.cur_pos)
+            q = self._qkv_rope_append(ly, x, self.seq_ids, self.cur_pos)
             att = torch.empty((b, nh * dv), dtype=torch.bfloat16, device=self.device)
             check(lib.sb_attn_decode(q.data_ptr(), q.stride(0), ly.cache_k.data_ptr(), ly.cache_v.data_ptr(),
                                      self.seq_lens.data_ptr(), b, nh, nkv, dk, dv, self.max_seq,

@@ -98,3 +98,31 @@ def test_attn_decode_key_group_edges(n_q, n_kv, dk, dv, n_split, shift):
         want = torch.einsum("hn,nhd->hd", p, vv)
         # fp32 sums, one rounding to bf16: half a step of 2^-8 of a value, and __expf's 2^-21
         assert float(((out[i].float() - want).abs() - 2.0 ** -8 * want.abs()).max()) < 1e-4
+
+
+@pytest.mark.parametrize("t,heads,rope,nope,dv,lora", [(1, 16, 64, 128, 128, 512), (5, 3, 16, 20, 12, 40)])
+def test_mla_append_and_strided_norm_give_the_bits_of_assembled_rows(t, heads, rope, nope, dv, lora):
+    torch.manual_seed(t + lora)
+    dk, s_max = rope + nope, t + 2
+    kv_a = torch.randn(t, lora + rope, device=DEV).to(BF)
+    kv = torch.randn(t, heads, nope + dv, device=DEV).to(BF)
+    q = torch.randn(t, heads * dk, device=DEV).to(BF)
+    w = torch.randn(lora, device=DEV).to(BF)
+    seq, pos = torch.zeros(t, dtype=torch.int32, device=DEV), torch.arange(t, dtype=torch.int32, device=DEV)
+    k = torch.cat([kv_a[:, lora:].unsqueeze(1).expand(t, heads, rope), kv[:, :, :nope]], dim=2).contiguous()
+    v = kv[:, :, nope:].contiguous()
+    caches = [[torch.zeros(1, s_max, heads, d, dtype=BF, device=DEV) for d in (dk, dv)] for _ in range(2)]
+    q1, q2 = q.clone(), q.clone()
+    check(lib.sb_rope_append(q1.data_ptr(), k.data_ptr(), v.data_ptr(), seq.data_ptr(), pos.data_ptr(), t, heads, heads,
+                             dk, dv, rope, 1.0e4, s_max, caches[0][0].data_ptr(), caches[0][1].data_ptr(), 0, 0, 0,
+                             _stream()), "sb_rope_append")
+    check(lib.sb_rope_append_mla(q2.data_ptr(), kv_a[:, lora:].data_ptr(), kv.data_ptr(), seq.data_ptr(), pos.data_ptr(),
+                                 t, heads, rope, nope, dv, 1.0e4, s_max, caches[1][0].data_ptr(),
+                                 caches[1][1].data_ptr(), heads * dk, lora + rope, heads * (nope + dv), _stream()),
+          "sb_rope_append_mla")
+    latent, a, b = kv_a[:, :lora].contiguous(), *(torch.empty(t, lora, dtype=BF, device=DEV) for _ in range(2))
+    check(lib.sb_add_rmsnorm(latent.data_ptr(), None, None, w.data_ptr(), 1e-6, t, lora, a.data_ptr(), _stream()), "norm")
+    check(lib.sb_rmsnorm_rows(kv_a.data_ptr(), lora + rope, w.data_ptr(), 1e-6, t, lora, b.data_ptr(), _stream()), "rows")
+    torch.cuda.synchronize()
+    assert torch.equal(q1, q2) and torch.equal(a, b)
+    assert all(torch.equal(x, y) for x, y in zip(*caches))
