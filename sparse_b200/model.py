@@ -215,8 +215,7 @@ class ShapedMoeModel:
 
     def _mlp(self, ly: _Layer, x: torch.Tensor) -> torch.Tensor:
         if ly.block is None:
-            out, _ = ops.grouped_swiglu(x, ly.dense_w13, ly.dense_w2, dense_rows=x.shape[0])
-            return out[:x.shape[0]]
+            return ops.dense_swiglu(x, ly.dense_w13, ly.dense_w2)
         out = torch.empty_like(x)
         ly.block.forward_device(x, out)
         if self.trace is not None:

@@ -120,6 +120,26 @@ def grouped_swiglu(rows: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor,
     return out, hbuf
 
 
+def dense_swiglu(rows: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor) -> torch.Tensor:
+    """One SwiGLU FFN over all rows: rows [T,H]; w13 [1,2I,H]; w2 [1,H,I] -> [T,H].
+
+    Up to `_lib.DECODE_MAX_TOKENS` rows the FFN is its weights' bytes, and the streaming
+    kernels read them with every SM; the tile kernel would walk the output in 256-row
+    tiles, for 10944 x 2048 eight of them in the down pass, on eight of the 74 CTA pairs
+    (26 + 52 us for 134 MB at one row)."""
+    t, h = rows.shape
+    i = w13.shape[1] // 2
+    if t > _lib.DECODE_MAX_TOKENS or h % 64 != 0 or i % 64 != 0:
+        return grouped_swiglu(rows, w13, w2, dense_rows=t)[0][:t]
+    hbuf = torch.empty((t, i), dtype=torch.bfloat16, device=rows.device)
+    out = torch.empty((t, h), dtype=torch.bfloat16, device=rows.device)
+    with torch.cuda.device(rows.device):
+        check(lib.sb_decode_experts(_ptr(rows), None, 1, None, None, None, None, None, h, i, 1, None, None,
+                                    _ptr(w13), _ptr(w2), None, i, t, _ptr(hbuf), _ptr(out), None, _stream(rows)),
+              "sb_decode_experts(dense)")
+    return out
+
+
 def combine(rows_out: torch.Tensor, slot_of_item: torch.Tensor, idx: torch.Tensor,
             shared_out: Optional[torch.Tensor], tokens: int,
             shared_scale: Optional[torch.Tensor] = None) -> torch.Tensor:

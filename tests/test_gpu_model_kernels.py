@@ -6,6 +6,7 @@ import math
 import pytest
 import torch
 
+from sparse_b200 import ops
 from sparse_b200._lib import lib, check
 
 pytestmark = pytest.mark.gpu
@@ -126,3 +127,17 @@ def test_mla_append_and_strided_norm_give_the_bits_of_assembled_rows(t, heads, r
     torch.cuda.synchronize()
     assert torch.equal(q1, q2) and torch.equal(a, b)
     assert all(torch.equal(x, y) for x, y in zip(*caches))
+
+
+@pytest.mark.parametrize("t", [1, 8, 9, 16, 17])
+def test_dense_swiglu_on_either_side_of_the_streaming_limit(t):
+    torch.manual_seed(t)
+    h, i = 256, 1216
+    x = torch.randn(t, h, device=DEV).to(BF)
+    w13 = (0.05 * torch.randn(1, 2 * i, h, device=DEV)).to(BF)
+    w2 = (0.05 * torch.randn(1, h, i, device=DEV)).to(BF)
+    got = ops.dense_swiglu(x, w13, w2).float()
+    want = ops.grouped_swiglu(x, w13, w2, dense_rows=t)[0].float()
+    # fp32 sums in another order: the two differ where a bf16 rounding falls the other way
+    assert got.shape == (t, h)
+    assert float((got - want).norm() / want.norm()) < 5e-3
