@@ -47,7 +47,7 @@ def test_rope_vectors_give_the_bits_of_single_elements(t, heads, dk, dv, rope_di
     torch.cuda.synchronize()
     for a, b in zip(*got):
         assert torch.equal(a, b)
-    assert torch.equal(got[0][2][0, 1:t].reshape(t - 1, -1), v[1:])
+    assert torch.equal(got[0][2][0, 1:t].flatten(), v[1:].flatten())
 
 
 @pytest.mark.parametrize("t,h,with_delta", [(3, 8, True), (2, 504, True), (1, 2056, False), (2, 16384, True)])
