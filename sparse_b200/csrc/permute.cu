@@ -8,7 +8,7 @@
 // an item is (number of items of smaller expert id) + (number of earlier items
 // of the same expert), which is what a stable sort by expert id yields.
 //
-// Four launches: count (per 128-item chunk histogram) -> scan (per-expert
+// Above kFusedMaxItems items four launches: count (per 128-item chunk histogram) -> scan (per-expert
 // prefix over chunks, expert offsets, tile table) -> scatter (ranks inside a
 // chunk by warp match) -> gather (one warp per output row, 16-byte vectors).
 // The gather is the only HBM-heavy part: it reads T*H*2 bytes (re-reads of a
@@ -134,73 +134,157 @@ permute_scatter_kernel(const int32_t *__restrict__ item_expert,
   }
 }
 
-// Count, scan and scatter in ONE CTA for up to kFusedMaxItems items (a 4096-token
-// batch with top-4 routing is 16384): each of the 32 warps owns a contiguous
-// range of items, histograms it in shared memory, the per-expert prefix over the
-// warps gives every range its base, and the same warp then ranks its items in
-// order.  Same result as the three-kernel path, two launches and their
-// scheduling gaps fewer; the workspace is not touched.
-constexpr int kFusedMaxItems = 32768;
+// Count, scan and scatter in ONE launch of one cluster, up to kFusedMaxItems items
+// (16384 tokens with top-8 routing are 131072).  Bound by latency, not by bytes: the
+// routed GEMM waits for it.  Each warp of the CS CTAs owns a contiguous range of
+// items and ranks them among its own in one pass (warp match, running counts in
+// shared memory), leaving the rank where the slot will go; the CTAs hand each other
+// their totals through distributed shared memory; one warp per CTA scans the
+// experts; the second pass only adds the base of (expert, warp range).  Loads run
+// eight rounds of 32 items ahead, so a round does not wait for its own.  Same result
+// as the three-kernel path; the workspace is not touched.
+// 16 warps per CTA whatever the item count, so that a few hundred items are one
+// round (one warp per 512 items took 9 us for 256, 15 us for 1800); not 32, so that
+// a CTA finds room on an SM beside a GEMM CTA of another stream.  Eight CTAs above
+// kOneCtaItems: one CTA took 66 us for 30000 items beside a GEMM.
+constexpr int kFusedMaxItems = 262144;
+constexpr int kFusedWarps = 16;
+constexpr int kFusedCtas = 8;
+constexpr int kOneCtaItems = 2048;
 
-__global__ void __launch_bounds__(1024)
+template <int CS>
+__global__ void __launch_bounds__(kFusedWarps * 32)
 permute_fused_kernel(const int32_t *__restrict__ item_expert, const __nv_bfloat16 *__restrict__ item_scale,
                      int n_items, int E, int tile_cap, int tile_rows, int32_t *__restrict__ expert_offsets,
                      int32_t *__restrict__ slot_of_item, int32_t *__restrict__ item_of_slot,
                      __nv_bfloat16 *__restrict__ slot_scale, int32_t *__restrict__ tile_table) {
   extern __shared__ int fused_smem[];
-  int *hist = fused_smem;                    // [nw][E] counts, then bases
-  const int nw = blockDim.x >> 5;            // warps in this CTA (1..32, fewer for few items)
-  int *offs = hist + nw * E;                 // [E+1]
+  int *hist = fused_smem;                    // [kFusedWarps][E] counts, then bases
+  int *offs = hist + kFusedWarps * E;        // [E+1]
   int *tile_start = offs + (E + 1);          // [E+1]
-  int *tot = tile_start + (E + 1);           // [E]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int per_warp = ((n_items + nw - 1) / nw + 31) & ~31;     // items per warp, multiple of 32
-  const int begin = warp * per_warp;
-  const int end = min(n_items, begin + per_warp);
-  for (int i = threadIdx.x; i < nw * E; i += blockDim.x) hist[i] = 0;
-  __syncthreads();
-  for (int i = begin + lane; i < end; i += 32) {
-    const int e = item_expert[i];
-    if (e >= 0 && e < E) atomicAdd(&hist[warp * E + e], 1);
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    int run = 0;
-    for (int w = 0; w < nw; ++w) { const int c = hist[w * E + e]; hist[w * E + e] = run; run += c; }
-    tot[e] = run;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int o = 0, ts = 0;
-    for (int e = 0; e < E; ++e) {
-      offs[e] = o; tile_start[e] = ts;
-      o += tot[e];
-      ts += (tot[e] + tile_rows - 1) / tile_rows;
-    }
-    offs[E] = o; tile_start[E] = ts;
-    tile_table[0] = ts < tile_cap ? ts : tile_cap;
-    tile_table[1] = o;
-    tile_table[2] = tile_rows; tile_table[3] = 0;
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e <= E; e += blockDim.x) expert_offsets[e] = offs[e];
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    const int nt = tile_start[e + 1] - tile_start[e];
-    for (int m = 0; m < nt; ++m) {
-      const int ti = tile_start[e] + m;
-      if (ti >= tile_cap) break;
-      int32_t *ent = tile_table + kTileHeaderInts + (size_t)ti * kTileEntryInts;
-      const int rb = offs[e] + m * tile_rows;
-      const int re = offs[e + 1] < rb + tile_rows ? offs[e + 1] : rb + tile_rows;
-      ent[0] = e; ent[1] = rb; ent[2] = re; ent[3] = 0;
-    }
-  }
-  // scatter: hist[warp][e] is now the number of items of e in earlier warps.
-  // Items are fetched eight rounds ahead so the loads overlap instead of each
-  // round waiting for its own.
+  int *cta_tot = tile_start + (E + 1);       // [CS][E] items of every CTA of the cluster
   constexpr int kBatch = 8;
+  pdl_wait();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t cta = 0;
+  if constexpr (CS > 1) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(cta));
+  constexpr int kWarps = CS * kFusedWarps;
+  const int per_warp = ((n_items + kWarps - 1) / kWarps + 31) & ~31;     // items per warp, multiple of 32
+  const int begin = min(n_items, ((int)cta * kFusedWarps + warp) * per_warp);
+  const int end = min(n_items, begin + per_warp);
+  int *mine = hist + warp * E;
+  for (int e = lane; e < E; e += 32) mine[e] = 0;
+  __syncwarp();
   for (int b0 = begin; b0 < end; b0 += 32 * kBatch) {
     int ev[kBatch];
+#pragma unroll
+    for (int r = 0; r < kBatch; ++r) {
+      const int i = b0 + r * 32 + lane;
+      ev[r] = i < end ? item_expert[i] : -1;
+    }
+#pragma unroll
+    for (int r = 0; r < kBatch; ++r) {
+      const int i = b0 + r * 32 + lane;
+      const int e = ev[r] >= 0 && ev[r] < E ? ev[r] : -1;
+      if (b0 + r * 32 >= end) break;         // (uniform over the warp)
+      const unsigned peers = __match_any_sync(0xffffffffu, e);
+      const int rank = __popc(peers & ((1u << lane) - 1u));
+      const int before = e >= 0 ? mine[e] : 0;
+      __syncwarp();
+      if (e >= 0 && rank == 0) mine[e] = before + __popc(peers);
+      __syncwarp();
+      if (i < end) slot_of_item[i] = before + rank;
+    }
+  }
+  if constexpr (CS > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // this CTA runs
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    int c[kFusedWarps], run = 0;
+#pragma unroll
+    for (int w = 0; w < kFusedWarps; ++w) c[w] = hist[w * E + e];
+#pragma unroll
+    for (int w = 0; w < kFusedWarps; ++w) { hist[w * E + e] = run; run += c[w]; }
+    cta_tot[cta * E + e] = run;
+  }
+  __syncthreads();
+  if constexpr (CS > 1) {
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    for (int i = threadIdx.x; i < CS * E; i += blockDim.x) {
+      const uint32_t to = (uint32_t)(i / E);
+      int *place = cta_tot + cta * E + (i - (int)to * E);
+      if (to == cta) continue;
+      uint32_t addr;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                   : "=r"(addr) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(place))), "r"(to));
+      asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(*place) : "memory");
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+  if (warp == 0) {
+    // lane l scans experts 8l .. 8l+7
+    constexpr int kPerLane = kMaxExperts / 32;
+    int cnt[kPerLane], rows = 0, tiles = 0;
+#pragma unroll
+    for (int i = 0; i < kPerLane; ++i) {
+      const int e = lane * kPerLane + i;
+      cnt[i] = 0;
+      if (e < E)
+        for (int c = 0; c < CS; ++c) cnt[i] += cta_tot[c * E + e];
+      rows += cnt[i];
+      tiles += (cnt[i] + tile_rows - 1) / tile_rows;
+    }
+    int o = rows, ts = tiles;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int po = __shfl_up_sync(0xffffffffu, o, off), pt = __shfl_up_sync(0xffffffffu, ts, off);
+      if (lane >= off) { o += po; ts += pt; }
+    }
+    if (lane == 31) {
+      offs[E] = o; tile_start[E] = ts;
+      if (cta == 0) {
+        tile_table[0] = ts < tile_cap ? ts : tile_cap;
+        tile_table[1] = o;
+        tile_table[2] = tile_rows; tile_table[3] = 0;
+      }
+    }
+    o -= rows; ts -= tiles;
+#pragma unroll
+    for (int i = 0; i < kPerLane; ++i) {
+      const int e = lane * kPerLane + i;
+      if (e < E) { offs[e] = o; tile_start[e] = ts; }
+      o += cnt[i];
+      ts += (cnt[i] + tile_rows - 1) / tile_rows;
+    }
+  }
+  __syncthreads();
+  // base of (expert, warp range): the expert's rows, the earlier CTAs' and the earlier warps' items
+  for (int i = threadIdx.x; i < kFusedWarps * E; i += blockDim.x) {
+    const int e = i % E;
+    int base = offs[e];
+    for (int c = 0; c < (int)cta; ++c) base += cta_tot[c * E + e];
+    hist[i] += base;
+  }
+  if (cta == 0) {
+    for (int e = threadIdx.x; e <= E; e += blockDim.x) expert_offsets[e] = offs[e];
+    for (int e = threadIdx.x; e < E; e += blockDim.x) {
+      const int nt = tile_start[e + 1] - tile_start[e];
+      for (int m = 0; m < nt; ++m) {
+        const int ti = tile_start[e] + m;
+        if (ti >= tile_cap) break;
+        int32_t *ent = tile_table + kTileHeaderInts + (size_t)ti * kTileEntryInts;
+        const int rb = offs[e] + m * tile_rows;
+        const int re = offs[e + 1] < rb + tile_rows ? offs[e + 1] : rb + tile_rows;
+        ent[0] = e; ent[1] = rb; ent[2] = re; ent[3] = 0;
+      }
+    }
+  }
+  // The gather's CTAs may take their places from here on, not earlier: waiting for
+  // the whole sort they would keep a GEMM CTA of another stream off their SMs.
+  pdl_launch_dependents();
+  __syncthreads();
+  for (int b0 = begin; b0 < end; b0 += 32 * kBatch) {
+    int ev[kBatch], rk[kBatch];
     __nv_bfloat16 sv[kBatch];
 #pragma unroll
     for (int r = 0; r < kBatch; ++r) {
@@ -208,22 +292,16 @@ permute_fused_kernel(const int32_t *__restrict__ item_expert, const __nv_bfloat1
       ev[r] = -1;
       if (i < end) {
         ev[r] = item_expert[i];
+        rk[r] = slot_of_item[i];             // this lane wrote it
         if (slot_scale != nullptr) sv[r] = item_scale[i];
       }
     }
 #pragma unroll
     for (int r = 0; r < kBatch; ++r) {
       const int i = b0 + r * 32 + lane;
-      int e = ev[r];
-      if (e < 0 || e >= E) e = -1;
-      const unsigned peers = __match_any_sync(0xffffffffu, e);
-      const int rank = __popc(peers & ((1u << lane) - 1u));
-      int slot = -1;
-      if (e >= 0) slot = offs[e] + hist[warp * E + e] + rank;
-      __syncwarp();
-      if (e >= 0 && rank == 0) hist[warp * E + e] += __popc(peers);
-      __syncwarp();
       if (i < end) {
+        const int e = ev[r];
+        const int slot = e >= 0 && e < E ? mine[e] + rk[r] : -1;
         slot_of_item[i] = slot;
         if (slot >= 0) {
           item_of_slot[slot] = i;
@@ -234,11 +312,34 @@ permute_fused_kernel(const int32_t *__restrict__ item_expert, const __nv_bfloat1
   }
 }
 
+template <int CS>
+cudaError_t launch_permute_fused(const int32_t *item_expert, const void *item_scale, int n_items, int E, int tile_cap,
+                                 int32_t *expert_offsets, int32_t *slot_of_item, int32_t *item_of_slot,
+                                 void *slot_scale, int32_t *tile_table, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(CS);
+  cfg.blockDim = dim3(kFusedWarps * 32);
+  cfg.dynamicSmemBytes = ((size_t)(kFusedWarps + CS) * E + 2 * (size_t)(E + 1)) * sizeof(int);    // at most 27 KB
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = CS; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = CS > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, permute_fused_kernel<CS>, item_expert, static_cast<const __nv_bfloat16 *>(item_scale),
+                            n_items, E, tile_cap, (int)sb_tile_rows(), expert_offsets, slot_of_item, item_of_slot,
+                            static_cast<__nv_bfloat16 *>(slot_scale), tile_table);
+}
+
 // One warp per output row.
 __global__ void __launch_bounds__(256)
 permute_gather_kernel(const uint4 *__restrict__ x, const int32_t *__restrict__ item_of_slot,
                       const int32_t *__restrict__ expert_offsets, int E, int items_per_row,
                       int vec_per_row, uint4 *__restrict__ out_rows) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int n_rows = expert_offsets[E];
   const int warps_total = gridDim.x * (blockDim.x >> 5);
@@ -279,28 +380,18 @@ int32_t launch_permute(const void *x, const int32_t *item_expert, const void *it
   int32_t *counts = static_cast<int32_t *>(ws);
   const int tile_cap = n_items / SB_TILE_M + E;
   if (n_items > 0 && n_items <= kFusedMaxItems) {
-    // one warp per 512 items: a decode step's handful of items is one warp's work
-    // At most 16 warps: measured on B200, 16384 items take the same 25 us with 16
-    // warps as with 32, and a 512-thread CTA still finds room on an SM that a
-    // GEMM CTA of another stream occupies (44 us there; a 1024-thread CTA waits
-    // for the GEMM to leave, 125 us).
-    int nw = (n_items + 511) / 512;
-    nw = nw < 1 ? 1 : (nw > 16 ? 16 : nw);
-    const size_t smem = ((size_t)nw * E + 2 * (size_t)(E + 1) + E) * sizeof(int);
-    if (smem > 48 * 1024)
-      SB_CUDA_CHECK(cudaFuncSetAttribute(permute_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem));
-    permute_fused_kernel<<<1, nw * 32, smem, stream>>>(
-        item_expert, static_cast<const __nv_bfloat16 *>(item_scale), n_items, E, tile_cap, sb_tile_rows(),
-        expert_offsets, slot_of_item, item_of_slot, static_cast<__nv_bfloat16 *>(slot_scale), tile_table);
+    const auto sort = n_items > kOneCtaItems ? launch_permute_fused<kFusedCtas> : launch_permute_fused<1>;
+    SB_CUDA_CHECK(sort(item_expert, item_scale, n_items, E, tile_cap, expert_offsets, slot_of_item, item_of_slot,
+                       slot_scale, tile_table, stream));
     SB_LAUNCH_CHECK();
     if (out_rows != nullptr) {
       int gblocks = (n_items + 7) / 8;
       const int max_blocks = sb_device_sm_count() * 8;
       if (gblocks > max_blocks) gblocks = max_blocks;
-      permute_gather_kernel<<<gblocks, 256, 0, stream>>>(
-          static_cast<const uint4 *>(x), item_of_slot, expert_offsets, E, items_per_row, H / 8,
-          static_cast<uint4 *>(out_rows));
+      SB_CUDA_CHECK(launch_pdl(permute_gather_kernel, dim3(gblocks), dim3(256), 0, stream,
+                               static_cast<const uint4 *>(x), static_cast<const int32_t *>(item_of_slot),
+                               static_cast<const int32_t *>(expert_offsets), E, items_per_row, H / 8,
+                               static_cast<uint4 *>(out_rows)));
       SB_LAUNCH_CHECK();
     }
     return SB_OK;
@@ -325,9 +416,10 @@ int32_t launch_permute(const void *x, const int32_t *item_expert, const void *it
       int gblocks = (n_items + rows_per_block - 1) / rows_per_block;
       int max_blocks = sb_device_sm_count() * 8;
       if (gblocks > max_blocks) gblocks = max_blocks;
-      permute_gather_kernel<<<gblocks, 256, 0, stream>>>(
-          static_cast<const uint4 *>(x), item_of_slot, expert_offsets, E, items_per_row, H / 8,
-          static_cast<uint4 *>(out_rows));
+      SB_CUDA_CHECK(launch_pdl(permute_gather_kernel, dim3(gblocks), dim3(256), 0, stream,
+                               static_cast<const uint4 *>(x), static_cast<const int32_t *>(item_of_slot),
+                               static_cast<const int32_t *>(expert_offsets), E, items_per_row, H / 8,
+                               static_cast<uint4 *>(out_rows)));
       SB_LAUNCH_CHECK();
     }
   }

@@ -1,0 +1,26 @@
+"""GPU: the routing kernels at the edges of their launch shapes."""
+import pytest
+import torch
+
+from oracle import moe_oracle as mo
+from sparse_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+DEV = torch.device("cuda:0")
+
+
+@pytest.mark.parametrize("n,e", [(1, 3), (31, 60), (2048, 60), (2049, 256), (4097, 7), (262144, 64), (262145, 64)])
+def test_expert_sort_at_its_size_limits(n, e):
+    """One warp's items, one CTA, the cluster of eight, the three-kernel path."""
+    torch.manual_seed(n)
+    ids = (torch.rand(n).pow(3) * e).to(torch.int32).clamp_(max=e - 1)
+    slot, item, offs = mo.expert_sorted_permutation(ids.view(n, 1), e)
+    p = ops.permute(torch.zeros(n, 8, dtype=torch.bfloat16, device=DEV), ids.to(DEV), e, 1)
+    assert torch.equal(p.expert_offsets.cpu().long(), offs)
+    assert torch.equal(p.slot_of_item.cpu().long()[:n], slot)
+    assert torch.equal(p.item_of_slot.cpu().long()[:n], item)
+    tt, want = p.tile_table.cpu(), []
+    for x in range(e):
+        want += [[x, b, min(b + 256, int(offs[x + 1])), 0] for b in range(int(offs[x]), int(offs[x + 1]), 256)]
+    assert int(tt[0]) == len(want) and tt[4:4 + 4 * len(want)].view(-1, 4).tolist() == want
