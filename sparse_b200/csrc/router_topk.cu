@@ -13,11 +13,13 @@
 // lane sums are combined by an xor-butterfly with offsets 16, 8, 4, 2, 1; the
 // bias is added in fp32 and the result is rounded once to the model dtype.
 //
-// Work split: one CTA owns TB tokens whose activations sit in shared memory;
-// each of its 8 warps streams pairs of router rows from L2 and dots them with
-// all TB tokens, so a weight row is fetched once per CTA.  HBM traffic is one
-// read of x plus the outputs; the kernel is bound by the fp32 FMA pipe
-// (2*T*E*H flops on CUDA cores), not by DRAM.
+// Work split: one CTA owns TB tokens whose activations sit in shared memory; each
+// of its 8 warps streams groups of RW router rows from L2 and dots them with all
+// TB tokens, so a weight row is fetched once per CTA.  HBM traffic is one read of
+// x plus the outputs; above a thousand tokens the kernel is bound by the fp32 FMA
+// pipe and the L2 reads of the router rows (2*T*E*H flops on CUDA cores), below by
+// latency: there a cluster of CS CTAs shares a token tile, each takes 1/CS of the
+// router rows and hands every token's logits to the CTA that finishes the token.
 #include "sb_common.cuh"
 
 namespace sb {
@@ -220,11 +222,34 @@ template <> struct Pair4<float> {
   }
 };
 
-template <typename IN, int TB>
+__device__ __forceinline__ uint32_t router_cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// a float into the same shared-memory place of CTA `rank` of this cluster
+__device__ __forceinline__ void store_to_cta(float *place, uint32_t rank, float v) {
+  uint32_t addr;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+               : "=r"(addr) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(place))), "r"(rank));
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+// all CTAs that share a token tile
+template <int CS>
+__device__ __forceinline__ void sync_tile() {
+  if constexpr (CS == 1) {
+    __syncthreads();
+  } else {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+}
+
+template <typename IN, int TB, int RW, int CS>
 __global__ void __launch_bounds__(kRouterThreads, 2)
 router_kernel(const IN *__restrict__ x, const IN *__restrict__ wg, const float *__restrict__ bias,
               const IN *__restrict__ wsg, int T, int H, int E, int K, int renorm, int fp32_logits,
-              int tb_eff, int32_t *__restrict__ out_idx, IN *__restrict__ out_w,
+              int32_t *__restrict__ out_idx, IN *__restrict__ out_w,
               void *__restrict__ out_logits, IN *__restrict__ out_shared) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int kVecPerGroup = sizeof(IN) == 2 ? 1 : 2;      // uint4 per 8 elements
@@ -234,122 +259,101 @@ router_kernel(const IN *__restrict__ x, const IN *__restrict__ wg, const float *
   const int NR = E + (wsg != nullptr ? 1 : 0);
   const int ldl = E + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t0 = blockIdx.x * tb_eff;      // this CTA's tokens: t0 .. t0 + tb_eff - 1 (tb_eff <= TB)
+  const int rank = CS == 1 ? 0 : (int)router_cluster_rank();
+  const int t0 = blockIdx.x / CS * TB;     // this tile's tokens: t0 .. t0 + TB - 1, zeros past the last
 
   // stage the activation tile
   const int vec_per_tok = G * kVecPerGroup;
-  for (int i = threadIdx.x; i < tb_eff * vec_per_tok; i += kRouterThreads) {
+  for (int i = threadIdx.x; i < TB * vec_per_tok; i += kRouterThreads) {
     int t = i / vec_per_tok, v = i - t * vec_per_tok;
     uint4 val = make_uint4(0, 0, 0, 0);
     if (t0 + t < T)
       val = __ldg(reinterpret_cast<const uint4 *>(x + (size_t)(t0 + t) * H) + v);
     sx[i] = val;
   }
-  __syncthreads();
+  sync_tile<CS>();
 
-  // Four router rows per warp pass: one shared-memory read of a token's 8
-  // activations feeds 32 multiply-adds, issued as 16 two-wide fp32 FMAs
-  // (`fma.rn.f32x2`: two independent IEEE FMAs per instruction, so the bits are
-  // those of scalar FMAs).  Each lane therefore keeps TWO partial sums per logit,
-  // one over the even and one over the odd elements of its groups.  The next
-  // step's weight vectors are fetched before the current step's math.
-  constexpr int RW = 4;
+  // RW router rows per warp pass: one shared-memory read of a token's 8 activations
+  // feeds 8 * RW multiply-adds, issued as two-wide fp32 FMAs (`fma.rn.f32x2`: two
+  // independent IEEE FMAs per instruction, so the bits are those of scalar FMAs).
+  // Each lane therefore keeps TWO partial sums per logit, one over the even and one
+  // over the odd elements of its groups.  AHEAD steps of weight vectors are fetched
+  // before their math: one step beside the current one where the math covers a
+  // fetch, several steps at once where it does not.
+  constexpr int AHEAD = TB >= 4 ? 1 : sizeof(IN) == 2 ? 4 : 2;
   const int steps = (G + 31) / 32;
   const int groups = (NR + RW - 1) / RW;
-  for (int grp = warp; grp < groups; grp += kRouterWarps) {
-    const IN *wp[RW];
+  const bool whole = (G & 31) == 0;        // a hidden size of whole 256-element steps needs no lane guards
+  for (int grp = rank * kRouterWarps + warp; grp < groups; grp += CS * kRouterWarps) {
+    const IN *wp[RW];                      // rows past the last read row 0's weights; their sums are never stored
 #pragma unroll
     for (int r = 0; r < RW; ++r) {
       const int row = grp * RW + r;
-      wp[r] = (row < E) ? wg + (size_t)row * H : ((row < NR) ? wsg : nullptr);
+      wp[r] = (row < E || row >= NR) ? wg + (size_t)(row < E ? row : 0) * H : wsg;
     }
     Acc2 acc[TB][RW];
 #pragma unroll
     for (int t = 0; t < TB; ++t)
 #pragma unroll
       for (int r = 0; r < RW; ++r) acc[t][r] = Acc2::zero();
-    uint4 cur[RW][kVecPerGroup], nxt[RW][kVecPerGroup];
-#pragma unroll
-    for (int r = 0; r < RW; ++r)
-#pragma unroll
-      for (int v = 0; v < kVecPerGroup; ++v) {
-        cur[r][v] = make_uint4(0, 0, 0, 0);
-        if (lane < G && wp[r] != nullptr)
-          cur[r][v] = __ldg(reinterpret_cast<const uint4 *>(wp[r] + (size_t)lane * 8) + v);
-      }
-    // Full token tile and a hidden size of whole 256-element steps (the usual
-    // case): the same arithmetic without the per-token and per-row guards.  Rows
-    // past the last one read row 0's weights; their sums are never stored.
-    if (TB < 8 && tb_eff == TB && (G & 31) == 0) {      // (the 8-token tile has no registers to spare for a second loop)
-      const IN *wq[RW];
-#pragma unroll
-      for (int r = 0; r < RW; ++r) wq[r] = wp[r] != nullptr ? wp[r] : wg;
-#pragma unroll
-      for (int r = 0; r < RW; ++r)
-#pragma unroll
-        for (int v = 0; v < kVecPerGroup; ++v)
-          cur[r][v] = __ldg(reinterpret_cast<const uint4 *>(wq[r] + (size_t)lane * 8) + v);
-#pragma unroll 1
-      for (int j = 0; j < steps; ++j) {
-        const int g = j * 32 + lane;
-        if (j + 1 < steps) {
-#pragma unroll
-          for (int r = 0; r < RW; ++r)
-#pragma unroll
-            for (int v = 0; v < kVecPerGroup; ++v)
-              nxt[r][v] = __ldg(reinterpret_cast<const uint4 *>(wq[r] + (size_t)(g + 32) * 8) + v);
-        }
-        Pair4<IN> w[RW];
-#pragma unroll
-        for (int r = 0; r < RW; ++r) w[r].load(&cur[r][0]);
-#pragma unroll
-        for (int t = 0; t < TB; ++t) {
-          Pair4<IN> xv;
-          xv.load(sx + ((size_t)t * G + g) * kVecPerGroup);
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int r = 0; r < RW; ++r) acc[t][r].fma(xv, w[r], i);
-        }
-#pragma unroll
-        for (int r = 0; r < RW; ++r)
-#pragma unroll
-          for (int v = 0; v < kVecPerGroup; ++v) cur[r][v] = nxt[r][v];
-      }
-    } else
-    for (int j = 0; j < steps; ++j) {
+    uint4 cur[AHEAD][RW][kVecPerGroup];
+    const auto fetch = [&](uint4 (&dst)[RW][kVecPerGroup], int j) {
       const int g = j * 32 + lane;
-      const int gn = g + 32;
 #pragma unroll
       for (int r = 0; r < RW; ++r)
 #pragma unroll
         for (int v = 0; v < kVecPerGroup; ++v) {
-          nxt[r][v] = make_uint4(0, 0, 0, 0);
-          if (gn < G && wp[r] != nullptr)
-            nxt[r][v] = __ldg(reinterpret_cast<const uint4 *>(wp[r] + (size_t)gn * 8) + v);
+          dst[r][v] = make_uint4(0, 0, 0, 0);
+          if (j < steps && (whole || g < G)) dst[r][v] = __ldg(reinterpret_cast<const uint4 *>(wp[r] + (size_t)g * 8) + v);
         }
-      if (g < G) {
-        Pair4<IN> w[RW];
+    };
+    const auto step = [&](const uint4 (&src)[RW][kVecPerGroup], int j) {
+      const int g = j * 32 + lane;
+      if (!whole && g >= G) return;
+      Pair4<IN> w[RW];
 #pragma unroll
-        for (int r = 0; r < RW; ++r) w[r].load(&cur[r][0]);
+      for (int r = 0; r < RW; ++r) w[r].load(&src[r][0]);
 #pragma unroll
-        for (int t = 0; t < TB; ++t) {
-          if (t < tb_eff) {
-            Pair4<IN> xv;
-            xv.load(sx + ((size_t)t * G + g) * kVecPerGroup);
+      for (int t = 0; t < TB; ++t) {
+        Pair4<IN> xv;
+        xv.load(sx + ((size_t)t * G + g) * kVecPerGroup);
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-              for (int r = 0; r < RW; ++r) acc[t][r].fma(xv, w[r], i);
-          }
-        }
+          for (int r = 0; r < RW; ++r) acc[t][r].fma(xv, w[r], i);
       }
+    };
+    if constexpr (AHEAD == 1) {
+      uint4 nxt[RW][kVecPerGroup];
+      fetch(cur[0], 0);
+#pragma unroll 1
+      for (int j = 0; j < steps; ++j) {
+        fetch(nxt, j + 1);
+        step(cur[0], j);
 #pragma unroll
-      for (int r = 0; r < RW; ++r)
+        for (int r = 0; r < RW; ++r)
 #pragma unroll
-        for (int v = 0; v < kVecPerGroup; ++v) cur[r][v] = nxt[r][v];
+          for (int v = 0; v < kVecPerGroup; ++v) cur[0][r][v] = nxt[r][v];
+      }
+    } else {
+#pragma unroll 1
+      for (int j = 0; j < steps; j += AHEAD) {
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) fetch(cur[u], j + u);
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u)
+          if (j + u < steps) step(cur[u], j + u);
+      }
     }
-    if (TB * RW < 32) {                 // (a full 32 would need every register the loop above holds)
+    const auto deliver = [&](int t, int row, float sum) {
+      if (row >= NR) return;
+      if (row < E && bias != nullptr) sum = __fadd_rn(sum, bias[row]);
+      // the shared gate's logit (row E) is always a model-dtype linear output
+      const float v = (fp32_logits && row < E) ? sum : Load8<IN>::round_model(sum);
+      if constexpr (CS == 1) slog[t * ldl + row] = v;
+      else store_to_cta(slog + t * ldl + row, t % CS, v);
+    };
+    if constexpr (TB * RW > 4) {
       // lane t*RW + r ends up with the logit of (token t, row r of this group)
       float part[32];
 #pragma unroll
@@ -358,33 +362,21 @@ router_kernel(const IN *__restrict__ x, const IN *__restrict__ wg, const float *
       for (int t = 0; t < TB; ++t)
 #pragma unroll
         for (int r = 0; r < RW; ++r) part[t * RW + r] = acc[t][r].lane_sum();
-      float sum = warp_sum_each(part, lane);
-      const int t = lane / RW, row = grp * RW + lane % RW;
-      if (t < tb_eff && row < NR) {
-        if (row < E && bias != nullptr) sum = __fadd_rn(sum, bias[row]);
-        // the shared gate's logit (row E) is always a model-dtype linear output
-        slog[t * ldl + row] = (fp32_logits && row < E) ? sum : Load8<IN>::round_model(sum);
-      }
+      const float sum = warp_sum_each(part, lane);
+      if (lane / RW < TB) deliver(lane / RW, grp * RW + lane % RW, sum);
     } else {
 #pragma unroll
-      for (int t = 0; t < TB; ++t) {
-        if (t < tb_eff) {
+      for (int t = 0; t < TB; ++t)
 #pragma unroll
-          for (int r = 0; r < RW; ++r) {
-            const int row = grp * RW + r;
-            float sum = butterfly_sum(acc[t][r].lane_sum());
-            if (lane == 0 && row < NR) {
-              if (row < E && bias != nullptr) sum = __fadd_rn(sum, bias[row]);
-              slog[t * ldl + row] = (fp32_logits && row < E) ? sum : Load8<IN>::round_model(sum);
-            }
-          }
+        for (int r = 0; r < RW; ++r) {
+          const float sum = butterfly_sum(acc[t][r].lane_sum());
+          if (lane == 0) deliver(t, grp * RW + r, sum);
         }
-      }
     }
   }
-  __syncthreads();
+  sync_tile<CS>();
 
-  for (int t = warp; t < tb_eff; t += kRouterWarps) {
+  for (int t = rank + CS * warp; t < TB; t += CS * kRouterWarps) {
     const int tok = t0 + t;
     if (tok >= T) continue;
     const float *lg = slog + t * ldl;
@@ -483,51 +475,54 @@ router_rows_kernel(const IN *__restrict__ x, const IN *__restrict__ wg, const fl
   }
 }
 
-template <typename IN, int TB>
-int32_t launch_router_tb(const void *x, const void *wg, const float *bias, const void *wsg, int T,
-                         int H, int E, int K, int renorm, int fp32_logits, int32_t *out_idx,
-                         void *out_w, void *out_logits, void *out_shared, cudaStream_t stream) {
-  const size_t smem_max = (size_t)TB * H * sizeof(IN) + (size_t)TB * (E + 1) * sizeof(float);
-  auto kern = router_kernel<IN, TB>;
-  if (smem_max > 48 * 1024)
-    SB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max));
-  // tokens per CTA: as few as keeps the grid within four CTAs per SM, so the
-  // last wave is full (4096 tokens on 148 SMs -> 7 per CTA, 586 CTAs)
-  const int slots = 4 * (sb_device_sm_count() > 0 ? sb_device_sm_count() : 148);
-  int tb_eff = (T + slots - 1) / slots;
-  if (tb_eff < 1) tb_eff = 1;
-  if (tb_eff > TB) tb_eff = TB;
-  int blocks = (T + tb_eff - 1) / tb_eff;
-  kern<<<blocks, kRouterThreads, smem_max, stream>>>(
-      static_cast<const IN *>(x), static_cast<const IN *>(wg), bias, static_cast<const IN *>(wsg),
-      T, H, E, K, renorm, fp32_logits, tb_eff, out_idx, static_cast<IN *>(out_w), out_logits,
-      static_cast<IN *>(out_shared));
+template <typename IN, int TB, int RW, int CS>
+int32_t launch_router_tile(const void *x, const void *wg, const float *bias, const void *wsg, int T,
+                           int H, int E, int K, int renorm, int fp32_logits, int32_t *out_idx,
+                           void *out_w, void *out_logits, void *out_shared, cudaStream_t stream) {
+  const size_t smem = (size_t)TB * H * sizeof(IN) + (size_t)TB * (E + 1) * sizeof(float);
+  auto kern = router_kernel<IN, TB, RW, CS>;
+  if (smem > 48 * 1024)
+    SB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // The largest shared-memory split, the one a GEMM CTA needs: the two can then share an SM.
+  SB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                     (int)cudaSharedmemCarveoutMaxShared));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((T + TB - 1) / TB * CS));
+  cfg.blockDim = dim3(kRouterThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = CS; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = CS > 1 ? 1 : 0;
+  SB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, static_cast<const IN *>(x), static_cast<const IN *>(wg), bias,
+                                   static_cast<const IN *>(wsg), T, H, E, K, renorm, fp32_logits, out_idx,
+                                   static_cast<IN *>(out_w), out_logits, static_cast<IN *>(out_shared)));
   SB_LAUNCH_CHECK();
   return SB_OK;
 }
 
+// Tile shapes.  Up to seven tokens per CTA (28 running sums of two per lane are what
+// the registers hold, and 30 KB of shared memory still fit beside a GEMM CTA of
+// another stream); fewer tokens per tile, and the router rows split over a cluster,
+// while that is what it takes to give every SM two CTAs (148 SMs):
+//   T <= 74    1 token,  2 rows a pass, 4 CTAs per tile    T <= 592   4 tokens, 2 CTAs
+//   T <= 296   2 tokens, 4 rows a pass, 2 CTAs             T <= 1036  7 tokens, 2 CTAs
+//   above      7 tokens, 1 CTA
+// A tile of a wide hidden size gives up tokens until it fits 100 KB.
 template <typename IN>
 int32_t launch_router_t(const void *x, const void *wg, const float *bias, const void *wsg, int T,
                         int H, int E, int K, int renorm, int fp32_logits, int32_t *out_idx,
                         void *out_w, void *out_logits, void *out_shared, cudaStream_t stream) {
-  // Fewer tokens per CTA when there are few tokens, so decode-sized calls still
-  // spread over the SMs; 16 per CTA at prefill sizes to amortise the weight reads.
-  const size_t tile8 = (size_t)8 * H * sizeof(IN) + 8 * (size_t)(E + 1) * 4;
-  // 7 when that is all a CTA takes anyway (4096 tokens over four CTAs per SM on
-  // 148 SMs): the tile is sized by the template, and the less shared memory a
-  // router CTA asks for, the more of the SM a GEMM CTA of another stream keeps
-  const int sms = sb_device_sm_count() > 0 ? sb_device_sm_count() : 148;
-  if (T >= 1024 && tile8 <= 100 * 1024 && (T + 4 * sms - 1) / (4 * sms) <= 7)
-    return launch_router_tb<IN, 7>(x, wg, bias, wsg, T, H, E, K, renorm, fp32_logits, out_idx,
-                                    out_w, out_logits, out_shared, stream);
-  if (T >= 1024 && tile8 <= 100 * 1024)
-    return launch_router_tb<IN, 8>(x, wg, bias, wsg, T, H, E, K, renorm, fp32_logits, out_idx,
-                                    out_w, out_logits, out_shared, stream);
-  if (T >= 256)
-    return launch_router_tb<IN, 4>(x, wg, bias, wsg, T, H, E, K, renorm, fp32_logits, out_idx,
-                                   out_w, out_logits, out_shared, stream);
-  return launch_router_tb<IN, 1>(x, wg, bias, wsg, T, H, E, K, renorm, fp32_logits, out_idx, out_w,
-                                 out_logits, out_shared, stream);
+  const int slots = 2 * (sb_device_sm_count() > 0 ? sb_device_sm_count() : 148);
+  const size_t row = (size_t)H * sizeof(IN) + (size_t)(E + 1) * sizeof(float), room = 100 * 1024;
+  auto launch = launch_router_tile<IN, 1, 2, 4>;
+  if (T > slots / 4 && 2 * row <= room) launch = launch_router_tile<IN, 2, 4, 2>;
+  if (T > slots && 4 * row <= room) launch = launch_router_tile<IN, 4, 4, 2>;
+  if (T > 2 * slots && 7 * row <= room) launch = launch_router_tile<IN, 7, 4, 2>;
+  if (T > 7 * slots / 2 && 7 * row <= room) launch = launch_router_tile<IN, 7, 4, 1>;
+  return launch(x, wg, bias, wsg, T, H, E, K, renorm, fp32_logits, out_idx, out_w, out_logits, out_shared, stream);
 }
 
 }  // namespace

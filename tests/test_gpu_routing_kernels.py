@@ -24,3 +24,22 @@ def test_expert_sort_at_its_size_limits(n, e):
     for x in range(e):
         want += [[x, b, min(b + 256, int(offs[x + 1])), 0] for b in range(int(offs[x]), int(offs[x + 1]), 256)]
     assert int(tt[0]) == len(want) and tt[4:4 + 4 * len(want)].view(-1, 4).tolist() == want
+
+
+@pytest.mark.parametrize("h,e,k,dtype", [(2048, 60, 4, torch.bfloat16), (264, 256, 8, torch.bfloat16),
+                                         (2048, 64, 6, torch.float32), (16384, 8, 2, torch.bfloat16)])
+def test_router_rows_do_not_depend_on_the_tile_shape(h, e, k, dtype):
+    """Every tile shape (tokens per CTA, CTAs per tile), ragged last tiles: the bits of one token alone."""
+    torch.manual_seed(h + e)
+    total = 1100
+    x = torch.randn(total, h, device=DEV).to(dtype)
+    wg, ws = (torch.randn(e, h, device=DEV) * 0.02).to(dtype), (torch.randn(h, device=DEV) * 0.02).to(dtype)
+    bias = torch.randn(e, device=DEV)
+    whole = ops.router_topk(x, wg, k, bias, ws)
+    for t in (1, 2, 73, 75, 147, 149, 295, 297, 591, 593, 887, 889, 1035, 1037):
+        part = ops.router_topk(x[:t].contiguous(), wg, k, bias, ws)
+        for a, b in zip(whole, part):
+            assert torch.equal(a[:t], b)
+    one = ops.router_topk(x[total - 1:].contiguous(), wg, k, bias, ws)
+    for a, b in zip(whole, one):
+        assert torch.equal(a[total - 1:], b)
