@@ -14,8 +14,8 @@
 //    (32 KB instead of 48 KB per CTA for the same flops), the tensor cores read
 //    the token half of the peer through distributed shared memory.  That cuts
 //    L2->SM traffic by a third, which is what capped the single-CTA kernel.
-//  * up to six 36 KB stages (one K step of a full tile, or two K steps of a tile
-//    of at most 32 tokens); TMEM holds two 128-lane x 256-column accumulators per
+//  * three 64 KB stages (two K steps of a full tile, or three of a tile of at most
+//    32 tokens) or up to six 36 KB stages (one K step, or two); TMEM holds two 128-lane x 256-column accumulators per
 //    CTA.  A launch may ask for fewer stages so that a CTA of another kernel
 //    (the router) fits on the SM beside it.
 //  * tile walk: by default table order with a fixed stride over the CTA pairs.
@@ -64,10 +64,12 @@ constexpr int kThreads = 320;         // producer warp, MMA warp, 8 epilogue war
 constexpr int kEpiWarps = 8;
 constexpr uint32_t kABytes = kRowsPerCta * kBlockK * 2;      // 16 KB
 constexpr uint32_t kLightTokBytes = 16 * kBlockK * 2;         // 2 KB: a 16-row token box of one K step
-// A stage holds one K step of a full tile (A 16 KB + B up to 16 KB) or, for a
-// light tile (at most 16 tokens per CTA), TWO K steps (A, A', then the two
-// 2 KB token boxes): half as many barrier round trips per weight byte, twice
-// the bytes in flight, which is what bounds a tile that is pure weight traffic.
+// A stage holds one K step of a full tile (A 16 KB + B up to 16 KB), or two of them
+// in 64 KB.  For a light tile (at most 16 tokens per CTA) it holds one K step more:
+// its weight boxes, then its 2 KB token boxes.  Fewer barrier round trips per
+// weight byte and more bytes in flight (162 KB of weights and rows in the three
+// 64 KB stages, against 108 KB with two K steps in each), which is what bounds a
+// tile that is pure weight traffic.
 constexpr uint32_t kStageBytes = 2 * kABytes + 2 * kLightTokBytes;   // one K step per stage (36 KB)
 constexpr uint32_t kSlabBytes = 2 * kABytes;                        // A + B of one K step of a full tile
 constexpr uint32_t kStageBytes2 = 2 * kSlabBytes;                   // two K steps per stage (64 KB)
@@ -81,6 +83,8 @@ constexpr uint32_t kTailBytes = 256 + 2 * kScatterTileBytes + kMaxSched * 2;   /
 __host__ __device__ constexpr uint32_t smem_bytes(int stages, uint32_t stage_bytes = kStageBytes, bool tail = true) {
   return (uint32_t)stages * stage_bytes + 1024 + (tail ? kTailBytes : 256u);
 }
+static_assert(3 * (kABytes + kLightTokBytes) <= kStageBytes2 && 2 * (kABytes + kLightTokBytes) <= kStageBytes,
+              "a light tile's stage");
 static_assert(smem_bytes(kStages) <= 232448 && smem_bytes(kStages2, kStageBytes2) <= 232448, "shared memory of a CTA");
 constexpr unsigned long long kWaitLimitNs = 2000000000ull;
 constexpr int kSlotSkip = -2;
@@ -301,6 +305,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   unsigned char *smem_al = smem_raw + (smem_base - smem_u32(smem_raw));
   const uint32_t stage_bytes_all = (uint32_t)n_stages * stage_bytes;
   const int slabs = stage_bytes == kStageBytes2 ? 2 : 1;            // K steps of a full tile per stage
+  const int light_steps = slabs + 1;                                // K steps of a light tile per stage
   const uint32_t bar_full = smem_base + stage_bytes_all;            // kStages  (used in the leader CTA)
   const uint32_t bar_empty = bar_full + 8 * kStages;               // kStages  (both CTAs)
   const uint32_t bar_tfull = bar_empty + 8 * kStages;              // 2        (both CTAs)
@@ -419,16 +424,16 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
           }
           continue;
         }
-        for (int kb = 0; kb < num_kb; kb += 2) {
+        for (int kb = 0; kb < num_kb; kb += light_steps) {
           if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) { ok = false; break; }
           const uint32_t full_leader = full_leader0 + 8 * stage;
           const uint32_t sa = smem_base + stage * stage_bytes;
-          const int steps = kb + 1 < num_kb ? 2 : 1;
+          const int steps = min(light_steps, num_kb - kb);
           if (cta == 0) mbar_expect_tx(bar_full + 8 * stage, 2 * steps * (kABytes + tok_bytes));
           for (int q = 0; q < steps; ++q)
             tma_pair_load_3d(sa + q * kABytes, &tm_w, full_leader, (kb + q) * kBlockK, wrow, ch.slot);
           for (int q = 0; q < steps; ++q)
-            tma_pair_load_2d(sa + 2 * kABytes + q * kLightTokBytes, tok_map, full_leader, (kb + q) * kBlockK, tok0);
+            tma_pair_load_2d(sa + light_steps * kABytes + q * kLightTokBytes, tok_map, full_leader, (kb + q) * kBlockK, tok0);
           if (++stage == n_stages) { stage = 0; phase ^= 1u; }
         }
       }
@@ -463,15 +468,15 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             if (++stage == n_stages) { stage = 0; phase ^= 1u; }
           }
         } else {
-          for (int kb = 0; kb < num_kb; kb += 2) {
+          for (int kb = 0; kb < num_kb; kb += light_steps) {
             if (!mbar_wait(bar_full + 8 * stage, phase, abort_flag)) { ok = false; break; }
             tc_fence_after();
             const uint32_t sa = smem_base + stage * stage_bytes;
-            const int steps = kb + 1 < num_kb ? 2 : 1;
+            const int steps = min(light_steps, num_kb - kb);
             for (int q = 0; q < steps; ++q) {
               const uint64_t adesc = umma_desc_sw128(sa + q * kABytes);
-              const uint64_t bdesc = umma_desc_sw128(sa + 2 * kABytes + q * kLightTokBytes);
-              tc_mma_pair_bf16_x4(d_tmem, adesc, bdesc, idesc, (uint32_t)(kb | q));
+              const uint64_t bdesc = umma_desc_sw128(sa + light_steps * kABytes + q * kLightTokBytes);
+              tc_mma_pair_bf16_x4(d_tmem, adesc, bdesc, idesc, (uint32_t)(kb + q));
             }
             tc_commit_pair(bar_empty + 8 * stage);
             if (++stage == n_stages) { stage = 0; phase ^= 1u; }
@@ -767,7 +772,7 @@ int32_t launch_pass(const CUtensorMap &tm_w, const CUtensorMap *tm_x, const int3
                     const unsigned long long *row_dst, int n_stages, uint32_t stage_bytes, cudaStream_t stream) {
   const int n_wtiles = (w_rows + kTileW - 1) / kTileW;
   const int dense_chunk = tile_table == nullptr ? dense_chunk_rows(dense_rows, n_wtiles, grid / 2) : kMaxN;
-  const int light_rows_per_cta = 16;      // tiles with at most this many tokens per CTA take two K steps per 36 KB stage
+  const int light_rows_per_cta = 16;      // tiles with at most this many tokens per CTA take one K step more per stage
   auto kern = pair_gemm_kernel<MODE>;
   const int mode_now = sched_mode();
   const bool tail = row_dst != nullptr || (tile_table != nullptr && mode_now != 0);

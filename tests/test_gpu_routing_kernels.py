@@ -43,3 +43,21 @@ def test_router_rows_do_not_depend_on_the_tile_shape(h, e, k, dtype):
     one = ops.router_topk(x[total - 1:].contiguous(), wg, k, bias, ws)
     for a, b in zip(whole, one):
         assert torch.equal(a[total - 1:], b)
+
+
+@pytest.mark.parametrize("h,i", [(64, 64), (128, 192), (192, 320), (256, 448), (448, 64)])
+@pytest.mark.parametrize("t", [1, 17, 32, 33])
+def test_light_tiles_of_any_depth(h, i, t):
+    """K steps that fill the last stage of a light tile once, twice or wholly."""
+    torch.manual_seed(h + i + t)
+    x = torch.randn(t, h, device=DEV).to(torch.bfloat16)
+    w13 = (torch.randn(1, 2 * i, h, device=DEV) * 0.1).to(torch.bfloat16)
+    w2 = (torch.randn(1, h, i, device=DEV) * 0.1).to(torch.bfloat16)
+    out, hid = ops.grouped_swiglu(x, w13, w2, dense_rows=t)
+    g, u = (x.float() @ w13[0, j::2].float().T for j in (0, 1))
+    bf = torch.bfloat16
+    want_h = (torch.nn.functional.silu(g.to(bf).float()).to(bf) * u.to(bf)).float()
+    # fp32 sums in another order move a bf16 rounding now and then: a few steps of 2^-8 of a value
+    assert float((hid[:t].float() - want_h).norm() / want_h.norm()) < 5e-3
+    want = hid[:t].float() @ w2[0].float().T
+    assert float((out[:t].float() - want).norm() / want.norm()) < 5e-3
