@@ -245,8 +245,12 @@ __device__ __forceinline__ void sync_tile() {
   }
 }
 
+// Registers: a GEMM CTA of another stream has ten warps of 96, three of them on two of
+// the four schedulers; 112 a thread is what leaves two router warps room beside them.
+// (At 128 the router waited for the GEMM to end: 4096 tokens 696 us per layer against
+// 680 us, 16384 tokens 2249 us against 2178 us.)
 template <typename IN, int TB, int RW, int CS>
-__global__ void __launch_bounds__(kRouterThreads, 2)
+__global__ void __launch_bounds__(kRouterThreads) __maxnreg__(sizeof(IN) == 2 ? 112 : 128)
 router_kernel(const IN *__restrict__ x, const IN *__restrict__ wg, const float *__restrict__ bias,
               const IN *__restrict__ wsg, int T, int H, int E, int K, int renorm, int fp32_logits,
               int32_t *__restrict__ out_idx, IN *__restrict__ out_w,
@@ -503,13 +507,13 @@ int32_t launch_router_tile(const void *x, const void *wg, const float *bias, con
   return SB_OK;
 }
 
-// Tile shapes.  Up to seven tokens per CTA (28 running sums of two per lane are what
-// the registers hold, and 30 KB of shared memory still fit beside a GEMM CTA of
-// another stream); fewer tokens per tile, and the router rows split over a cluster,
+// Tile shapes.  Up to six tokens per CTA (24 running sums of two per lane are what the
+// registers hold, and 26 KB of shared memory still fit beside a GEMM CTA of another
+// stream); fewer tokens per tile, and the router rows split over a cluster,
 // while that is what it takes to give every SM two CTAs (148 SMs):
 //   T <= 74    1 token,  2 rows a pass, 4 CTAs per tile    T <= 592   4 tokens, 2 CTAs
-//   T <= 296   2 tokens, 4 rows a pass, 2 CTAs             T <= 1036  7 tokens, 2 CTAs
-//   above      7 tokens, 1 CTA
+//   T <= 296   2 tokens, 4 rows a pass, 2 CTAs             T <= 888   6 tokens, 2 CTAs
+//   above      6 tokens, 1 CTA
 // A tile of a wide hidden size gives up tokens until it fits 100 KB.
 template <typename IN>
 int32_t launch_router_t(const void *x, const void *wg, const float *bias, const void *wsg, int T,
@@ -520,8 +524,8 @@ int32_t launch_router_t(const void *x, const void *wg, const float *bias, const 
   auto launch = launch_router_tile<IN, 1, 2, 4>;
   if (T > slots / 4 && 2 * row <= room) launch = launch_router_tile<IN, 2, 4, 2>;
   if (T > slots && 4 * row <= room) launch = launch_router_tile<IN, 4, 4, 2>;
-  if (T > 2 * slots && 7 * row <= room) launch = launch_router_tile<IN, 7, 4, 2>;
-  if (T > 7 * slots / 2 && 7 * row <= room) launch = launch_router_tile<IN, 7, 4, 1>;
+  if (T > 2 * slots && 6 * row <= room) launch = launch_router_tile<IN, 6, 4, 2>;
+  if (T > 3 * slots && 6 * row <= room) launch = launch_router_tile<IN, 6, 4, 1>;
   return launch(x, wg, bias, wsg, T, H, E, K, renorm, fp32_logits, out_idx, out_w, out_logits, out_shared, stream);
 }
 
