@@ -590,9 +590,12 @@ int32_t sb_moe_layer_forward(const sb_moe_layer *layer, int32_t *status, void *s
  *                  and merged by a second kernel; ws needs
  *                  sb_attn_decode_workspace_bytes.  Built for (dk,dv) =
  *                  (128,128), (192,128), (64,64).
+ * sb_argmax_rows   out[b] = index of the largest of the V logits of row b, the first
+ *                  one among equals, NaN above every number.
  */
 int32_t sb_add_rmsnorm(void *residual, const void *delta, const void *delta2, const void *weight, float eps,
                        int32_t T, int32_t H, void *out, void *stream);
+int32_t sb_argmax_rows(const void *logits, int32_t B, int32_t V, int64_t *out, void *stream);
 int32_t sb_rmsnorm_rows(const void *rows, int32_t row_stride, const void *weight, float eps, int32_t T, int32_t H,
                         void *out, void *stream);
 int32_t sb_rope_append_mla(void *q, const void *k_pe, const void *kv, const int32_t *seq_of_token,

@@ -496,6 +496,78 @@ int32_t launch_attn_decode(const __nv_bfloat16 *q, int q_stride, const __nv_bflo
   return SB_OK;
 }
 
+// Greedy token of every row of logits: the index of the largest value, the first
+// one among equals, NaN above every number (torch.argmax's rules).  A cluster of
+// eight CTAs per row: each reads its eighth of the vocabulary as 16-byte vectors and
+// the leader takes the best of the eight through distributed shared memory.
+// Latency-bound: one row of 102400 is 200 KB (a library reduction over an fp32 copy
+// of the row took 25 + 5 us, on one CTA).
+constexpr int kArgmaxThreads = 512;
+constexpr int kArgmaxCtas = 8;
+
+// values as keys in their order; index in the low half so that of equal values the first wins
+__device__ __forceinline__ unsigned long long argmax_key(uint32_t bf16_bits, uint32_t index) {
+  const uint32_t mag = bf16_bits & 0x7fffu;
+  uint32_t ord = bf16_bits & 0x8000u ? 0x8000u - mag : 0x8000u + mag;       // -0 and +0 give the same
+  if (mag > 0x7f80u) ord = 0x10000u;                                        // NaN
+  return ((unsigned long long)ord << 32) | (0xffffffffu - index);
+}
+__device__ __forceinline__ unsigned long long key_max(unsigned long long a, unsigned long long b) { return a > b ? a : b; }
+
+__global__ void __cluster_dims__(kArgmaxCtas, 1, 1) __launch_bounds__(kArgmaxThreads)
+argmax_rows_kernel(const __nv_bfloat16 *__restrict__ logits, int V, int vec, int64_t *__restrict__ out) {
+  __shared__ unsigned long long best_of_warp[kArgmaxThreads / 32];
+  __shared__ unsigned long long best_of_cta[kArgmaxCtas];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int row = blockIdx.x / kArgmaxCtas;
+  uint32_t rank;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  const unsigned short *src = reinterpret_cast<const unsigned short *>(logits) + (size_t)row * V;
+  unsigned long long best = 0;
+  if (vec) {
+    const uint4 *v = reinterpret_cast<const uint4 *>(src);
+#pragma unroll 4
+    for (int i = rank * kArgmaxThreads + threadIdx.x; i < V / 8; i += kArgmaxCtas * kArgmaxThreads) {
+      const uint4 q = __ldg(v + i);
+      const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        best = key_max(best, argmax_key(w[k] & 0xffffu, 8 * i + 2 * k));
+        best = key_max(best, argmax_key(w[k] >> 16, 8 * i + 2 * k + 1));
+      }
+    }
+  } else {
+    for (int i = rank * kArgmaxThreads + threadIdx.x; i < V; i += kArgmaxCtas * kArgmaxThreads)
+      best = key_max(best, argmax_key(src[i], i));
+  }
+#pragma unroll
+  for (int off = 16; off >= 1; off >>= 1) best = key_max(best, __shfl_xor_sync(0xffffffffu, best, off));
+  if ((threadIdx.x & 31) == 0) best_of_warp[threadIdx.x >> 5] = best;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    best = threadIdx.x < kArgmaxThreads / 32 ? best_of_warp[threadIdx.x] : 0;
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) best = key_max(best, __shfl_xor_sync(0xffffffffu, best, off));
+  }
+  // (the first arrive also says that every CTA of the cluster has started)
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (threadIdx.x == 0) {
+    uint32_t addr;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;"
+                 : "=r"(addr) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(best_of_cta + rank))));
+    asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"(best) : "memory");
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (rank == 0 && threadIdx.x == 0) {
+#pragma unroll
+    for (int c = 0; c < kArgmaxCtas; ++c) best = key_max(best, best_of_cta[c]);
+    out[row] = (int64_t)(0xffffffffu - (uint32_t)best);
+  }
+}
+
 }  // namespace
 }  // namespace sb
 
@@ -562,6 +634,17 @@ int32_t sb_rope_append_mla(void *q, const void *k_pe, const void *kv, const int3
                      RopeSource{rest, kv_stride, nope_dim + dv}, RopeSource{rest + nope_dim, kv_stride, nope_dim + dv},
                      seq_of_token, pos_of_token, T, n_heads, n_heads, dk, dv, rope_dim, theta, s_max, cache_k, cache_v,
                      static_cast<cudaStream_t>(stream));
+}
+
+int32_t sb_argmax_rows(const void *logits, int32_t B, int32_t V, int64_t *out, void *stream) {
+  if (B < 0 || V < 1 || B > (1 << 24)) return fail(SB_E_INVALID_ARG, "sb_argmax_rows: bad shape (B=%d V=%d)", B, V);
+  if (B == 0) return SB_OK;
+  if (!logits || !out) return fail(SB_E_INVALID_ARG, "sb_argmax_rows: null pointer");
+  SB_CUDA_CHECK(launch_pdl(argmax_rows_kernel, dim3(B * kArgmaxCtas), dim3(kArgmaxThreads), 0,
+                           static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16 *>(logits), V,
+                           V % 8 == 0 && aligned(logits, 16) ? 1 : 0, out));
+  SB_LAUNCH_CHECK();
+  return SB_OK;
 }
 
 size_t sb_attn_decode_workspace_bytes(int32_t B, int32_t n_q, int32_t dv, int32_t n_split) {

@@ -296,7 +296,7 @@ class ShapedMoeModel:
             delta = self._mlp(ly, x2)
         normed = self._norm(resid, delta, self.final_norm)
         logits = F.linear(normed, self.lm_head)
-        self.cur_ids.copy_(torch.argmax(logits.float(), dim=-1))
+        check(lib.sb_argmax_rows(logits.data_ptr(), b, cfg.vocab, self.cur_ids.data_ptr(), self._s()), "sb_argmax_rows")
         self.cur_pos.add_(1)
 
     def decode_step(self, use_graph: bool = True) -> torch.Tensor:

@@ -141,3 +141,20 @@ def test_dense_swiglu_on_either_side_of_the_streaming_limit(t):
     # fp32 sums in another order: the two differ where a bf16 rounding falls the other way
     assert got.shape == (t, h)
     assert float((got - want).norm() / want.norm()) < 5e-3
+
+
+@pytest.mark.parametrize("b,v", [(1, 1), (3, 4096), (2, 102400), (8, 151936), (2, 1003)])
+def test_argmax_rows_is_torch_argmax(b, v):
+    torch.manual_seed(v)
+    logits = (torch.randn(b, v, device=DEV) * 0.5).to(BF)          # coarse values: many ties
+    logits[0, v // 2] = -0.0
+    if b > 1:
+        logits[1] = -float("inf")
+        logits[1, v - 1] = float("nan") if v == 4096 else -float("inf")
+    if b > 2:
+        logits[2] = 0.0
+        logits[2, ::2] = -0.0
+    ids = torch.empty(b, dtype=torch.int64, device=DEV)
+    check(lib.sb_argmax_rows(logits.data_ptr(), b, v, ids.data_ptr(), _stream()), "sb_argmax_rows")
+    torch.cuda.synchronize()
+    assert torch.equal(ids.cpu(), torch.argmax(logits.float().cpu(), dim=-1))
