@@ -574,6 +574,8 @@ int32_t sb_moe_layer_forward(const sb_moe_layer *layer, int32_t *status, void *s
  *                  k_stride, v_stride: elements between consecutive tokens
  *                  (0 = densely packed), so q, k, v may be column slices of
  *                  one fused projection output.
+ * sb_decode_linear out [T,N] = bf16(x [T,K] . w [N,K]^T + bias [N] (may be NULL)) for
+ *                  T <= SB_DECODE_MAX_TOKENS, fp32 sums, K a multiple of 32.
  * sb_rmsnorm_rows  out [T,H] = weight * bf16(row * rsqrt(mean(row^2) + eps)) of rows
  *                  that lie `row_stride` elements apart (column slices of a
  *                  projection output); the rows themselves are not written.
@@ -596,6 +598,8 @@ int32_t sb_moe_layer_forward(const sb_moe_layer *layer, int32_t *status, void *s
 int32_t sb_add_rmsnorm(void *residual, const void *delta, const void *delta2, const void *weight, float eps,
                        int32_t T, int32_t H, void *out, void *stream);
 int32_t sb_argmax_rows(const void *logits, int32_t B, int32_t V, int64_t *out, void *stream);
+int32_t sb_decode_linear(const void *x, const void *w, const void *bias, int32_t T, int32_t N, int32_t K, void *out,
+                         void *stream);
 int32_t sb_rmsnorm_rows(const void *rows, int32_t row_stride, const void *weight, float eps, int32_t T, int32_t H,
                         void *out, void *stream);
 int32_t sb_rope_append_mla(void *q, const void *k_pe, const void *kv, const int32_t *seq_of_token,

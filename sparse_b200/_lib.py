@@ -94,6 +94,7 @@ SIGNATURES: Dict[str, Tuple[object, list]] = {
     "sb_rope_append": (i32, [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, C.c_float, i32, vp, vp, i32, i32, i32,
                              vp]),
     "sb_argmax_rows": (i32, [vp, i32, i32, vp, vp]),
+    "sb_decode_linear": (i32, [vp, vp, vp, i32, i32, i32, vp, vp]),
     "sb_rmsnorm_rows": (i32, [vp, i32, vp, C.c_float, i32, i32, vp, vp]),
     "sb_rope_append_mla": (i32, [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, C.c_float, i32, vp, vp, i32, i32, i32,
                                  vp]),

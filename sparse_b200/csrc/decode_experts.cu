@@ -291,6 +291,55 @@ decode_down_kernel(const __nv_bfloat16 *__restrict__ hbuf, const int32_t *__rest
   }
 }
 
+// out = bf16(x . W^T + bias) for at most 16 rows: the projections around the experts
+// in a decode step.  Block task = (8/ks_n) x 16 weight rows over ks_n slices of K.
+// Bound by the weights' bytes, 8 to 25 MB: a few microseconds, of which the start is
+// a good part, so the first weight lines of a task are asked into L2 while the
+// launch before this one ends (a prefetch reads nothing: L2 is where a write of
+// that launch would land too).
+__global__ void __launch_bounds__(kThreads, 2)
+decode_linear_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ w,
+                     const __nv_bfloat16 *__restrict__ bias, int T, int N, int K, int ks_n,
+                     __nv_bfloat16 *__restrict__ out) {
+  __shared__ float red[kWarps][8][32];
+  pdl_launch_dependents();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, c = lane & 3;
+  const int rg = warp / ks_n, ks = warp % ks_n;
+  const int n0 = (blockIdx.x * (kWarps / ks_n) + rg) * 16;
+  const int chunks = K / 32, per = (chunks + ks_n - 1) / ks_n;
+  const int ch0 = min(chunks, ks * per), ch1 = min(chunks, ch0 + per);
+  const __nv_bfloat16 *row_lo = w + (size_t)min(n0 + g, N - 1) * K + c * 8;
+  const __nv_bfloat16 *row_hi = w + (size_t)min(n0 + 8 + g, N - 1) * K + c * 8;
+  // lane c of a row asks for every fourth of its 128-byte lines (two chunks each)
+  for (int ch = ch0 + 2 * c; ch < min(ch1, ch0 + 16); ch += 8) {
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(row_lo + (size_t)ch * 32));
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(row_hi + (size_t)ch * 32));
+  }
+  pdl_wait();
+  const __nv_bfloat16 *tok[2];
+#pragma unroll
+  for (int nt = 0; nt < 2; ++nt) tok[nt] = x + (size_t)min(nt * 8 + g, T - 1) * K + c * 8;
+  float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+  if (T > 8) stream_rows<2>(row_lo, row_hi, tok, ch0, ch1, acc);
+  else stream_rows<1>(row_lo, row_hi, tok, ch0, ch1, acc);
+  reduce_k_slices(acc, warp, lane, ks, ks_n, red);
+  if (ks != 0) return;
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    const int n = n0 + half * 8 + g;
+    if (n >= N) continue;
+    const float b = bias != nullptr ? __bfloat162float(bias[n]) : 0.f;
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int t = nt * 8 + 2 * c + i;
+        if (t < T) out[(size_t)t * N + n] = __float2bfloat16_rn(acc[nt][half * 2 + i] + b);
+      }
+  }
+}
+
 }  // namespace
 
 int32_t launch_decode_experts(const void *x, const int32_t *item_of_slot, int items_per_row,
@@ -346,3 +395,24 @@ int32_t launch_decode_experts(const void *x, const int32_t *item_of_slot, int it
 }
 
 }  // namespace sb
+
+extern "C" int32_t sb_decode_linear(const void *x, const void *w, const void *bias, int32_t T, int32_t N, int32_t K,
+                                    void *out, void *stream) {
+  using namespace sb;
+  if (T < 0 || T > SB_DECODE_MAX_TOKENS || N < 1 || K < 32 || K % 32 != 0)
+    return fail(SB_E_INVALID_ARG, "sb_decode_linear: need 0<=T<=%d, N>=1, K%%32==0 (T=%d N=%d K=%d)",
+                SB_DECODE_MAX_TOKENS, T, N, K);
+  if (T == 0) return SB_OK;
+  if (!x || !w || !out) return fail(SB_E_INVALID_ARG, "sb_decode_linear: null pointer");
+  if (!aligned(x, 16) || !aligned(w, 16)) return fail(SB_E_INVALID_ARG, "sb_decode_linear: x and w must be 16-byte aligned");
+  // as many K slices as keep the launch within one round of two CTAs per SM
+  const int sms = sb_device_sm_count() > 0 ? sb_device_sm_count() : 148;
+  int ks = kWarps;
+  while (ks > 1 && (N * ks + 127) / 128 > 2 * sms) ks /= 2;
+  SB_CUDA_CHECK(launch_pdl(decode_linear_kernel, dim3((N * ks + 127) / 128), dim3(kThreads), 0,
+                           static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16 *>(x),
+                           static_cast<const __nv_bfloat16 *>(w), static_cast<const __nv_bfloat16 *>(bias), T, N, K, ks,
+                           static_cast<__nv_bfloat16 *>(out)));
+  SB_LAUNCH_CHECK();
+  return SB_OK;
+}

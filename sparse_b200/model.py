@@ -186,7 +186,7 @@ class ShapedMoeModel:
         if cfg.attention == "mla":
             nope, rope, lora = dk - cfg.rope_dim, cfg.rope_dim, cfg.kv_lora_rank
             if t <= _lib.DECODE_MAX_TOKENS:      # a few rows: one launch over both weights
-                q_kva = F.linear(x, ly.wq_kva)                         # q per head: [rope | nope]
+                q_kva = ops.linear(x, ly.wq_kva)                        # q per head: [rope | nope]
                 q, kv_a = q_kva[:, :nh * dk], q_kva[:, nh * dk:]
             else:
                 q, kv_a = F.linear(x, ly.wq), F.linear(x, ly.wkv_a)
@@ -194,14 +194,14 @@ class ShapedMoeModel:
             c_kv = torch.empty((t, lora), dtype=x.dtype, device=x.device)
             check(lib.sb_rmsnorm_rows(latent.data_ptr(), latent.stride(0), ly.kv_norm.data_ptr(), cfg.rms_eps, t, lora,
                                       c_kv.data_ptr(), self._s()), "sb_rmsnorm_rows")
-            kv = F.linear(c_kv, ly.wkv_b)                              # per head: [nope | v]
+            kv = ops.linear(c_kv, ly.wkv_b)                             # per head: [nope | v]
             check(lib.sb_rope_append_mla(q.data_ptr(), k_pe.data_ptr(), kv.data_ptr(), seq_of_token.data_ptr(),
                                          pos_of_token.data_ptr(), t, nh, rope, nope, dv, cfg.rope_theta, self.max_seq,
                                          ly.cache_k.data_ptr(), ly.cache_v.data_ptr(), q.stride(0), k_pe.stride(0),
                                          kv.stride(0), self._s()), "sb_rope_append_mla")
             return q
         # column slices of the fused projection: the kernels take the token stride
-        qkv = F.linear(x, ly.wqkv, ly.bqkv)
+        qkv = ops.linear(x, ly.wqkv, ly.bqkv)
         q, k, v = qkv[:, :nh * dk], qkv[:, nh * dk:nh * dk + nkv * dk], qkv[:, nh * dk + nkv * dk:]
         check(lib.sb_rope_append(q.data_ptr(), k.data_ptr(), v.data_ptr(), seq_of_token.data_ptr(),
                                  pos_of_token.data_ptr(), t, nh, nkv, dk, dv, cfg.rope_dim, cfg.rope_theta,
@@ -252,7 +252,7 @@ class ShapedMoeModel:
             att = F.scaled_dot_product_attention(qh, kh, vh, attn_mask=mask, is_causal=mask is None,
                                                  scale=1.0 / math.sqrt(dk))
             att = att[..., :dv].transpose(1, 2).reshape(t, nh * dv)
-            attn_out = F.linear(att, ly.wo)
+            attn_out = ops.linear(att, ly.wo)
             x2 = self._norm(resid, attn_out, ly.ln2)
             delta = self._mlp(ly, x2)
         check(lib.sb_add_rmsnorm(resid.data_ptr(), delta.data_ptr(), None, None, cfg.rms_eps, t, cfg.hidden, None,
@@ -291,7 +291,7 @@ class ShapedMoeModel:
                                      self.seq_lens.data_ptr(), b, nh, nkv, dk, dv, self.max_seq,
                                      1.0 / math.sqrt(dk), self.n_split, self.attn_ws.data_ptr(),
                                      self.attn_ws.numel(), att.data_ptr(), self._s()), "sb_attn_decode")
-            attn_out = F.linear(att, ly.wo)
+            attn_out = ops.linear(att, ly.wo)
             x2 = self._norm(resid, attn_out, ly.ln2)
             delta = self._mlp(ly, x2)
         normed = self._norm(resid, delta, self.final_norm)

@@ -140,6 +140,20 @@ def dense_swiglu(rows: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor) -> tor
     return out
 
 
+def linear(rows: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """rows [T,K] . weight [N,K]^T (+ bias): the weight-streaming kernel up to
+    `_lib.DECODE_MAX_TOKENS` rows (8 MB of weights: 7 us through the library at one
+    to eight rows, most of them not spent on the bytes), the library's GEMM above."""
+    (t, k), n = rows.shape, weight.shape[0]
+    if t > _lib.DECODE_MAX_TOKENS or k % 32 != 0 or not rows.is_contiguous():
+        return torch.nn.functional.linear(rows, weight, bias)
+    out = torch.empty((t, n), dtype=torch.bfloat16, device=rows.device)
+    with torch.cuda.device(rows.device):
+        check(lib.sb_decode_linear(_ptr(rows), _ptr(weight), _ptr(bias), t, n, k, _ptr(out), _stream(rows)),
+              "sb_decode_linear")
+    return out
+
+
 def combine(rows_out: torch.Tensor, slot_of_item: torch.Tensor, idx: torch.Tensor,
             shared_out: Optional[torch.Tensor], tokens: int,
             shared_scale: Optional[torch.Tensor] = None) -> torch.Tensor:

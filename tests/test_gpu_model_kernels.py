@@ -158,3 +158,17 @@ def test_argmax_rows_is_torch_argmax(b, v):
     check(lib.sb_argmax_rows(logits.data_ptr(), b, v, ids.data_ptr(), _stream()), "sb_argmax_rows")
     torch.cuda.synchronize()
     assert torch.equal(ids.cpu(), torch.argmax(logits.float().cpu(), dim=-1))
+
+
+@pytest.mark.parametrize("t", [1, 8, 9, 16, 17])
+@pytest.mark.parametrize("n,k,with_bias", [(1, 32, True), (130, 96, False), (2048, 2048, True), (6144, 512, False)])
+def test_linear_on_either_side_of_the_streaming_limit(t, n, k, with_bias):
+    torch.manual_seed(t + n)
+    x = torch.randn(t, k, device=DEV).to(BF)
+    w = (torch.randn(n, k, device=DEV) / math.sqrt(k)).to(BF)
+    b = torch.randn(n, device=DEV).to(BF) if with_bias else None
+    got = ops.linear(x, w, b)
+    want = x.double() @ w.double().T + (b.double() if with_bias else 0.0)
+    # fp32 sums of at most 2048 products of order 1 / sqrt(k), one rounding to bf16
+    assert got.shape == (t, n)
+    assert float(((got.double() - want).abs() - 2.0 ** -8 * want.abs()).max()) < 1e-4
