@@ -154,9 +154,11 @@ class ShapedMoeModel:
                                         process_group=process_group, owner=owner)
             self.layers.append(ly)
         # enough key splits for about six CTAs per SM: a CTA streams its keys with
-        # a few hundred bytes in flight per warp, so bandwidth comes from CTA count
+        # a few hundred bytes in flight per warp, so bandwidth comes from CTA count;
+        # but 64 keys a split at the longest, two turns of a CTA's 16 key groups: more
+        # splits of fewer keys only lengthen the merge
         sms = max(1, int(lib.sb_device_sm_count()) or 148)
-        self.n_split = max(1, min(64, (6 * sms + batch * nh - 1) // (batch * nh)))
+        self.n_split = max(1, min(64, (6 * sms + batch * nh - 1) // (batch * nh), (max_seq + 63) // 64))
         ws = lib.sb_attn_decode_workspace_bytes(batch, nh, dv, self.n_split)
         self.attn_ws = torch.empty((ws,), dtype=torch.uint8, device=device)
         # decode-step state advanced by the graph itself
