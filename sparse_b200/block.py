@@ -96,18 +96,21 @@ class B200MoeBlock:
                 self._warm = True
             self.last_launches = self._ep.last_launches
             return res
+        return self._forward_local(x, out)
+
+    _warm = False
+
+    def _forward_local(self, x: torch.Tensor, out: Optional[torch.Tensor], first_row: int = 0) -> torch.Tensor:
         if self.use_graphs and self._warm and x.shape[0] <= self.runner.max_tokens:
-            return self._forward_graphed_local(x, out)
-        res, _, _, _ = self.runner.forward(x, out)
+            return self._forward_graphed_local(x, out, first_row)
+        res, _, _, _ = self.runner.forward(x, out, first_row)
         self._warm = True
         self.last_launches = self.runner.last_launches
         return res
 
-    _warm = False
-
-    def _forward_graphed_local(self, x: torch.Tensor, out: Optional[torch.Tensor]) -> torch.Tensor:
-        dst = self.runner.out[:x.shape[0]] if out is None else out
-        key = (x.data_ptr(), x.shape[0], dst.data_ptr())
+    def _forward_graphed_local(self, x: torch.Tensor, out: Optional[torch.Tensor], first_row: int = 0) -> torch.Tensor:
+        dst = self.runner.out[first_row:first_row + x.shape[0]] if out is None else out
+        key = (x.data_ptr(), x.shape[0], dst.data_ptr(), first_row)
         ent = self._graphs.get(key)
         if ent is None:
             if len(self._graphs) >= 32:
@@ -118,7 +121,7 @@ class B200MoeBlock:
             graph = torch.cuda.CUDAGraph()
             with torch.cuda.stream(cap):
                 with torch.cuda.graph(graph, stream=cap, capture_error_mode="thread_local"):
-                    self.runner.forward(x, dst)
+                    self.runner.forward(x, dst, first_row)
             stream.wait_stream(cap)
             ent = (graph, self.runner.last_launches, x, dst)
             self._graphs[key] = ent
@@ -134,10 +137,48 @@ class B200MoeBlock:
             self._x_stage = torch.empty((max(t, self.runner.max_tokens), h), dtype=torch.bfloat16,
                                         device=self.device)
         xd = self._x_stage[:t]
-        xd.copy_(x_host, non_blocking=True)
-        out = self.forward_device(xd)
-        out_host.copy_(out, non_blocking=True)
-        torch.cuda.current_stream(self.device).synchronize()
+        stream = torch.cuda.current_stream(self.device)
+        parts = self._host_parts(t)
+        if parts == 1:
+            xd.copy_(x_host, non_blocking=True)
+            out = self.forward_device(xd)
+            out_host.copy_(out, non_blocking=True)
+            stream.synchronize()
+            return
+        # Part i + 1 comes in and part i - 1 goes out while part i is in the layer (a
+        # row's result does not depend on the rows around it).
+        if self._copy_lanes is None:
+            self._copy_lanes = torch.cuda.Stream(device=self.device), torch.cuda.Stream(device=self.device)
+        inward, outward = self._copy_lanes
+        inward.wait_stream(stream)
+        launches = 0
+        rows = [t * i // parts // 16 * 16 for i in range(parts)] + [t]
+        arrived = []
+        with torch.cuda.stream(inward):
+            for r0, r1 in zip(rows, rows[1:]):
+                xd[r0:r1].copy_(x_host[r0:r1], non_blocking=True)
+                arrived.append(inward.record_event())
+        for r0, r1, there in zip(rows, rows[1:], arrived):
+            stream.wait_event(there)
+            out = self._forward_local(xd[r0:r1], None, r0)
+            launches += self.last_launches
+            outward.wait_stream(stream)
+            with torch.cuda.stream(outward):
+                out_host[r0:r1].copy_(out, non_blocking=True)
+        self.last_launches = launches
+        stream.wait_stream(outward)
+        stream.synchronize()
+
+    _copy_lanes = None
+
+    def _host_parts(self, tokens: int) -> int:
+        """Parts a host batch is passed in.  Splitting hides all copies but the first
+        part's in and the last part's out (75 ns a row each way), and costs the layer
+        time that two half batches take longer than one: from 3072 rows the copies
+        win (a batch below streams the expert weights twice for little)."""
+        if self._ep is not None or tokens < 3072 or tokens > self.runner.max_tokens:
+            return 1
+        return max(2, tokens // 4096)
 
     def host_pipeline(self, depth: int = 3) -> "HostPipeline":
         """A queue for host-resident batches: copy-in, layer and copy-out of

@@ -145,16 +145,21 @@ class LayerRunner:
                                       dtype=torch.float32 if self.fp32_logits else torch.bfloat16,
                                       device=dev)
 
-    def forward(self, x: torch.Tensor, out: Optional[torch.Tensor] = None):
+    def forward(self, x: torch.Tensor, out: Optional[torch.Tensor] = None, first_row: int = 0):
         """x [T,H] bf16 on the layer's device -> (out [T,H], topk_idx, topk_w, logits).
-        Returned tensors are views of buffers this runner reuses on the next call."""
+        Returned tensors are views of buffers this runner reuses on the next call.
+        `first_row`: where the rows' results go in those buffers, for a batch that is
+        passed in parts (its rows must fit in `max_tokens`)."""
         w = self.w
         if x.dtype != torch.bfloat16 or not x.is_cuda or not x.is_contiguous():
             raise RuntimeError("LayerRunner.forward needs a contiguous CUDA bf16 tensor")
         t = x.shape[0]
+        if first_row and first_row + t > self.max_tokens:
+            raise RuntimeError("rows %d..%d of a runner for %d" % (first_row, first_row + t, self.max_tokens))
         if t > self.max_tokens:
             self._reserve(t)
-        dst = self.out[:t] if out is None else out
+        rows = slice(first_row, first_row + t)
+        dst = self.out[rows] if out is None else out
         L = MoeLayer()
         L.T, L.H, L.E, L.K, L.I, L.I_shared = t, w.hidden, w.num_experts, self.top_k, w.inter, w.shared_inter
         L.renorm, L.n_slots = int(self.renorm), w.n_slots
@@ -168,16 +173,17 @@ class LayerRunner:
         L.shared_w13 = w.shared_w13.data_ptr() if w.shared_w13 is not None else None
         L.shared_w2 = w.shared_w2.data_ptr() if w.shared_w2 is not None else None
         L.out = dst.data_ptr()
-        L.logits = self.logits.data_ptr() if self.logits is not None else None
-        L.topk_idx, L.topk_w = self.topk_idx.data_ptr(), self.topk_w.data_ptr()
+        logits = self.logits[rows] if self.logits is not None else None
+        idx, weight = self.topk_idx[rows], self.topk_w[rows]
+        L.logits = logits.data_ptr() if logits is not None else None
+        L.topk_idx, L.topk_w = idx.data_ptr(), weight.data_ptr()
         L.ws, L.ws_bytes = self._ws_ptr, self._ws_bytes
         with torch.cuda.device(w.device):
             stream = torch.cuda.current_stream(w.device).cuda_stream
             check(lib.sb_moe_layer_forward(C.byref(L), self.status.data_ptr(), stream),
                   "sb_moe_layer_forward")
         self.last_launches = int(lib.sb_last_launch_count())
-        logits = self.logits[:t] if self.logits is not None else None
-        return dst, self.topk_idx[:t], self.topk_w[:t], logits
+        return dst, idx, weight, logits
 
     def check_status(self) -> None:
         """Host-synchronising check of the device status word (tests, debug)."""
