@@ -364,7 +364,14 @@ int32_t launch_decode_experts(const void *x, const int32_t *item_of_slot, int it
   // K slices per row group (measured on B200: 2 slices for 64 chunks of 32
   // elements, 1 for 44, 4 for 176 beat finer splits by up to 8 % at 8 tokens)
   auto slices = [](int k) { const int ch = k / 32; return ch > 128 ? 4 : ch > 48 ? 2 : 1; };
-  const int ks1 = slices(H), ks2_routed = slices(I), ks2_shared = slices(I_sh > 0 ? I_sh : I);
+  const int ks1 = slices(H);
+  int ks2_routed = slices(I), ks2_shared = slices(I_sh > 0 ? I_sh : I);
+  // The down pass of one token has 128 tasks for 296 CTAs, and which SMs the busy ones
+  // land on is chance: twice the K slices, twice the tasks (751 -> 734 us per step of
+  // nine DeepSeek-shaped layers at one token).
+  const long down_tasks = (tile_table ? (long)T * items_per_row : 0) * ((H * ks2_routed + 127) / 128) +
+                          (shared_w13 ? (H * ks2_shared + 127) / 128 : 0);
+  if (2 * down_tasks <= grid) { ks2_routed *= 2; ks2_shared = ks2_shared < 8 ? ks2_shared * 2 : 8; }
   // (Splitting K finer at one or two tokens, so that the 352 pass-1 / 128 pass-2
   // tasks of a single token spread over all CTAs in several small rounds, was
   // measured slower on B200: 50 us against 45 us per layer at one token.  The
