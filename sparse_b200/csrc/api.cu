@@ -38,7 +38,7 @@ static inline size_t up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 // host threads from interleaving their records on the shared events.
 struct SideLane {
   cudaStream_t stream = nullptr;
-  cudaEvent_t fork = nullptr, mid = nullptr, join = nullptr;
+  cudaEvent_t fork = nullptr, mid = nullptr, join = nullptr, started = nullptr;
 };
 static std::recursive_mutex g_side_mu;
 static SideLane g_side[64];
@@ -56,15 +56,15 @@ static int32_t create_side_lane(int dev) {
   if (l.stream != nullptr) return SB_OK;
   cudaStream_t st = nullptr;
   SB_CUDA_CHECK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-  cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
-  for (int i = 0; i < 3; ++i) {
+  cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
+  for (int i = 0; i < 4; ++i) {
     if (cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming) != cudaSuccess) {
       for (int j = 0; j < i; ++j) cudaEventDestroy(ev[j]);
       cudaStreamDestroy(st);
       return fail(SB_E_CUDA, "sb_init: cannot create the layer driver's events");
     }
   }
-  l.fork = ev[0]; l.mid = ev[1]; l.join = ev[2];
+  l.fork = ev[0]; l.mid = ev[1]; l.join = ev[2]; l.started = ev[3];
   l.stream = st;
   return SB_OK;
 }
@@ -96,10 +96,10 @@ int32_t launch_grouped_swiglu_any(const void *rows, const int32_t *tile_table, i
                                   const void *w13, const void *w2, const int32_t *slot_of_expert,
                                   const void *row_scale, int R_cap, int H, int I, int S, void *hbuf,
                                   void *out, int32_t *status, cudaStream_t stream, int max_pairs = 0,
-                                  int passes = 3, int stages = 0) {
+                                  int passes = 3, int stages = 0, cudaEvent_t started = nullptr) {
   return launch_grouped_swiglu_pair(rows, tile_table, dense_rows, w13, w2, slot_of_expert, row_scale,
                                     R_cap, H, I, S, hbuf, out, status, 0, max_pairs, nullptr, stream, passes,
-                                    stages);
+                                    stages, started);
 }
 
 // Carves the caller's workspace; the same walk gives the required size.
@@ -192,7 +192,11 @@ static int32_t layer_forward_large(const sb_moe_layer *L, const LayerScratch &s,
   if (beside)
     rc_shared = launch_grouped_swiglu_any(L->x, nullptr, T, L->shared_w13, L->shared_w2, nullptr, nullptr, T, H, Is,
                                           1, s.shared_h, s.shared_out, status, stream,
-                                          split ? shared_pairs() : 0, 1, kStagesBesideRouter);
+                                          split ? shared_pairs() : 0, 1, kStagesBesideRouter,
+                                          split ? nullptr : lane->started);
+  // The router's CTAs fit beside the GEMM's, not the other way round: where both want
+  // every SM the GEMM takes its places first.
+  if (beside && !split && rc_shared == SB_OK) SB_CUDA_CHECK(cudaStreamWaitEvent(side, lane->started, 0));
   rc = SB_OK;
   if (beside)
     rc = launch_router(L->x, L->router_w, L->router_bias, L->shared_gate_w, T, H, E, K, L->renorm, SB_DTYPE_BF16,

@@ -769,20 +769,30 @@ template <int MODE>
 int32_t launch_pass(const CUtensorMap &tm_w, const CUtensorMap *tm_x, const int32_t *tile_table, int dense_rows,
                     const int32_t *slot_of_expert, const void *row_scale, void *out, int ld_out, int w_rows,
                     int num_kb, int n_slots, int32_t *status, int grid, int skip_rows_upto,
-                    const unsigned long long *row_dst, int n_stages, uint32_t stage_bytes, cudaStream_t stream) {
+                    const unsigned long long *row_dst, int n_stages, uint32_t stage_bytes, cudaStream_t stream,
+                    cudaEvent_t started = nullptr) {
   const int n_wtiles = (w_rows + kTileW - 1) / kTileW;
   const int dense_chunk = tile_table == nullptr ? dense_chunk_rows(dense_rows, n_wtiles, grid / 2) : kMaxN;
   const int light_rows_per_cta = 16;      // tiles with at most this many tokens per CTA take one K step more per stage
   auto kern = pair_gemm_kernel<MODE>;
   const int mode_now = sched_mode();
   const bool tail = row_dst != nullptr || (tile_table != nullptr && mode_now != 0);
-  kern<<<grid, kThreads, smem_bytes(n_stages, stage_bytes, tail), stream>>>(tm_w, tm_x[0], tm_x[1], tm_x[2], tile_table, dense_rows,
-                                                        slot_of_expert,
-                                                        static_cast<const __nv_bfloat16 *>(row_scale),
-                                                        static_cast<__nv_bfloat16 *>(out), ld_out, w_rows, num_kb,
-                                                        n_slots, status, skip_rows_upto, dense_chunk, light_rows_per_cta,
-                                                        row_dst, n_stages, mode_now,
-                                                        g_dense_group.load(std::memory_order_relaxed), stage_bytes);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem_bytes(n_stages, stage_bytes, tail);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeLaunchCompletionEvent;
+  attr[0].val.launchCompletionEvent.event = started;
+  attr[0].val.launchCompletionEvent.flags = 0;
+  cfg.attrs = attr;
+  cfg.numAttrs = started != nullptr ? 1 : 0;
+  SB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tm_w, tm_x[0], tm_x[1], tm_x[2], tile_table, dense_rows, slot_of_expert,
+                                   static_cast<const __nv_bfloat16 *>(row_scale), static_cast<__nv_bfloat16 *>(out),
+                                   ld_out, w_rows, num_kb, n_slots, status, skip_rows_upto, dense_chunk,
+                                   light_rows_per_cta, row_dst, n_stages, mode_now,
+                                   g_dense_group.load(std::memory_order_relaxed), stage_bytes));
   SB_LAUNCH_CHECK();
   return SB_OK;
 }
@@ -816,11 +826,12 @@ int32_t set_gemm_tuning(const char *key, int value) {
 // of `out`.  `passes`: 1 = gate/up + SwiGLU only, 2 = down only (hbuf already
 // holds the intermediate rows), 3 = both.  `stages` in [2, 6] is the depth of
 // the shared-memory pipeline (0 = 5, which leaves room on the SM for a router CTA).
+// `started`: an event that fires when every CTA of the gate/up pass has its SM.
 int32_t launch_grouped_swiglu_pair(const void *rows, const int32_t *tile_table, int dense_rows, const void *w13,
                                    const void *w2, const int32_t *slot_of_expert, const void *row_scale,
                                    int R_cap, int H, int I, int S, void *hbuf, void *out, int32_t *status,
                                    int skip_rows_upto, int max_pairs, const unsigned long long *row_dst,
-                                   cudaStream_t stream, int passes, int stages) {
+                                   cudaStream_t stream, int passes, int stages, cudaEvent_t started) {
   if (H < kBlockK || I < kBlockK || H % kBlockK != 0 || I % kBlockK != 0)
     return fail(SB_E_UNSUPPORTED, "sb_grouped_swiglu: H and I must be multiples of %d (H=%d I=%d)", kBlockK, H, I);
   if (R_cap <= 0 || S < 1) return fail(SB_E_INVALID_ARG, "sb_grouped_swiglu: R_cap=%d S=%d", R_cap, S);
@@ -858,7 +869,8 @@ int32_t launch_grouped_swiglu_pair(const void *rows, const int32_t *tile_table, 
   if (max_pairs > 0 && 2 * max_pairs < grid) grid = 2 * max_pairs;     // leave the other SMs to a concurrent launch
   if (passes & 1) {
     rc = launch_pass<kModeSwiglu>(tm_w13, tm_x, tile_table, dense_rows, slot_of_expert, nullptr, hbuf, I, 2 * I,
-                                  H / kBlockK, S, status, grid, skip_rows_upto, nullptr, stages, stage_bytes, stream);
+                                  H / kBlockK, S, status, grid, skip_rows_upto, nullptr, stages, stage_bytes, stream,
+                                  started);
     if (rc != SB_OK) return rc;
   }
   if (!(passes & 2)) return SB_OK;

@@ -106,7 +106,7 @@ int32_t launch_grouped_swiglu_pair(const void *rows, const int32_t *tile_table, 
                                    const void *row_scale, int R_cap, int H, int I, int S,
                                    void *hbuf, void *out, int32_t *status, int skip_rows_upto, int max_pairs,
                                    const unsigned long long *row_dst, cudaStream_t stream, int passes = 3,
-                                   int stages = 0);
+                                   int stages = 0, cudaEvent_t started = nullptr);
 int32_t set_gemm_tuning(const char *key, int value);
 int32_t set_ep_tuning(const char *key, int value);       // SB_E_UNSUPPORTED: not one of its keys
 int32_t launch_decode_experts(const void *x, const int32_t *item_of_slot, int items_per_row,
