@@ -77,6 +77,11 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return *reinterpret_cast<uint32_t *>(&v);
 }
 
+// Decode-sized layer pass: from this many tokens the shared expert's gate/up tasks run
+// beside the expert sort (97 against 100 us at 8 tokens, 138 against 147 us at 16;
+// at one token the loaded memory system makes the sort the longer part: 48 against 46.5 us).
+constexpr int kSharedBesideSortTokens = 2;
+
 // Tile table layout shared by sb_permute and the grouped GEMM.
 constexpr int kTileHeaderInts = 4;   // [0] = number of row tiles
 constexpr int kTileEntryInts = 4;    // expert, row_begin, row_end, 0
@@ -115,7 +120,7 @@ int32_t launch_decode_experts(const void *x, const int32_t *item_of_slot, int it
                               void *y, const void *shared_w13, const void *shared_w2,
                               const void *shared_scale, int I_sh, int T, void *shared_h, void *shared_out,
                               int32_t *status, int ctas_per_sm, int max_rows, const void *shared_x,
-                              const unsigned long long *row_dst, cudaStream_t stream);
+                              const unsigned long long *row_dst, cudaStream_t stream, bool shared_early = false);
 int32_t launch_combine(const void *rows_out, const int32_t *slot_of_item, const int32_t *idx,
                        const void *shared_out, const void *shared_scale, int T, int H, int K, void *out,
                        cudaStream_t stream);
