@@ -142,13 +142,13 @@ static LayerScratch carve(char *base, int T, int H, int E, int K, int I, int I_s
 // nothing from the routing and its down pass only the scalar gate, so with a
 // shared expert the work is split over two streams:
 //
-//   caller's stream   shared gate/up (5-stage pipeline) . shared down .        . routed GEMMs . combine
+//   caller's stream   shared gate/up . shared down .        . routed GEMMs . combine
 //   side stream       router . count/scan/scatter/gather ^(mid)        ^(join)
 //
-// The gate/up launch goes first and takes one CTA per SM with a pipeline one
-// stage shorter than usual; what it leaves free on each SM (shared memory,
-// registers) is what one router CTA needs, so the router's CUDA-core dot
-// products run under the tensor-core pass instead of in front of it.  Up to
+// The gate/up launch goes first and takes one CTA per SM; what it leaves free on
+// each SM (shared memory, registers) is what one router CTA needs, so the router's
+// CUDA-core dot products run under the tensor-core pass instead of in front of it
+// (16384 tokens: 640 us for the two, 500 + 220 us one after the other).  Up to
 // split_tokens() rows, where both GEMMs stream weights and neither fills the
 // machine, the routed GEMM follows on the side stream too and the two share
 // the SMs by grid size.  Without a shared expert everything runs in order on
@@ -200,7 +200,7 @@ static int32_t layer_forward_large(const sb_moe_layer *L, const LayerScratch &s,
   rc = SB_OK;
   if (beside)
     rc = launch_router(L->x, L->router_w, L->router_bias, L->shared_gate_w, T, H, E, K, L->renorm, SB_DTYPE_BF16,
-                       L->router_fp32_logits, L->topk_idx, L->topk_w, L->logits, shared_scale, side);
+                       L->router_fp32_logits, L->topk_idx, L->topk_w, L->logits, shared_scale, side, true);
   SB_CUDA_CHECK(cudaEventRecord(lane->mid, side));
   if (rc == SB_OK)
     rc = launch_permute(L->x, L->topk_idx, L->topk_w, T * K, K, H, E, s.permute_ws, s.permute_ws_bytes, s.xs,
@@ -210,8 +210,8 @@ static int32_t layer_forward_large(const sb_moe_layer *L, const LayerScratch &s,
                                    H, I, L->n_slots, s.hbuf, s.y, status, side, all_pairs - shared_pairs());
   SB_CUDA_CHECK(cudaEventRecord(lane->join, side));
   // The shared expert's down pass leaves the scalar gate to the combine kernel, so
-  // it does not wait for the router (which takes 190 us instead of 73 us while it
-  // shares the SMs with the gate/up pass).
+  // it does not wait for the router (three times as long beside the gate/up pass as
+  // alone).
   if (rc_shared == SB_OK)
     rc_shared = launch_grouped_swiglu_any(L->x, nullptr, T, L->shared_w13, L->shared_w2, nullptr, nullptr, T,
                                           H, Is, 1, s.shared_h, s.shared_out, status, stream,

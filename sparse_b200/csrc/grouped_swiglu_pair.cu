@@ -288,8 +288,8 @@ struct Sched {
 };
 
 // The gate/up instance is held to 96 registers per thread (the "two CTAs per SM"
-// of its launch bounds says only that): with 320 threads that leaves an SM the
-// 32 K registers a router CTA needs beside it.
+// of its launch bounds says only that): three of its ten warps on a scheduler then
+// leave the room for two warps of a router CTA (112 registers a thread) beside them.
 template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, MODE == kModeScale ? 1 : 2)
 pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,

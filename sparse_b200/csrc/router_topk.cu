@@ -245,12 +245,8 @@ __device__ __forceinline__ void sync_tile() {
   }
 }
 
-// Registers: a GEMM CTA of another stream has ten warps of 96, three of them on two of
-// the four schedulers; 112 a thread is what leaves two router warps room beside them.
-// (At 128 the router waited for the GEMM to end: 4096 tokens 696 us per layer against
-// 680 us, 16384 tokens 2249 us against 2178 us.)
-template <typename IN, int TB, int RW, int CS>
-__global__ void __launch_bounds__(kRouterThreads) __maxnreg__(sizeof(IN) == 2 ? 112 : 128)
+template <typename IN, int TB, int RW, int CS, int REGS>
+__global__ void __launch_bounds__(kRouterThreads) __maxnreg__(REGS)
 router_kernel(const IN *__restrict__ x, const IN *__restrict__ wg, const float *__restrict__ bias,
               const IN *__restrict__ wsg, int T, int H, int E, int K, int renorm, int fp32_logits,
               int32_t *__restrict__ out_idx, IN *__restrict__ out_w,
@@ -479,12 +475,12 @@ router_rows_kernel(const IN *__restrict__ x, const IN *__restrict__ wg, const fl
   }
 }
 
-template <typename IN, int TB, int RW, int CS>
+template <typename IN, int TB, int RW, int CS, int REGS = 128>
 int32_t launch_router_tile(const void *x, const void *wg, const float *bias, const void *wsg, int T,
                            int H, int E, int K, int renorm, int fp32_logits, int32_t *out_idx,
                            void *out_w, void *out_logits, void *out_shared, cudaStream_t stream) {
   const size_t smem = (size_t)TB * H * sizeof(IN) + (size_t)TB * (E + 1) * sizeof(float);
-  auto kern = router_kernel<IN, TB, RW, CS>;
+  auto kern = router_kernel<IN, TB, RW, CS, REGS>;
   if (smem > 48 * 1024)
     SB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   // The largest shared-memory split, the one a GEMM CTA needs: the two can then share an SM.
@@ -507,25 +503,31 @@ int32_t launch_router_tile(const void *x, const void *wg, const float *bias, con
   return SB_OK;
 }
 
-// Tile shapes.  Up to six tokens per CTA (24 running sums of two per lane are what the
-// registers hold, and 26 KB of shared memory still fit beside a GEMM CTA of another
-// stream); fewer tokens per tile, and the router rows split over a cluster,
-// while that is what it takes to give every SM two CTAs (148 SMs):
+// Tile shapes.  Up to seven tokens per CTA (28 running sums of two per lane are what 128
+// registers hold); fewer tokens per tile, and the router rows split over a cluster, while
+// that is what it takes to give every SM two CTAs (148 SMs):
 //   T <= 74    1 token,  2 rows a pass, 4 CTAs per tile    T <= 592   4 tokens, 2 CTAs
-//   T <= 296   2 tokens, 4 rows a pass, 2 CTAs             T <= 888   6 tokens, 2 CTAs
-//   above      6 tokens, 1 CTA
+//   T <= 296   2 tokens, 4 rows a pass, 2 CTAs             T <= 1036  7 tokens, 2 CTAs
+//   above      7 tokens, 1 CTA
 // A tile of a wide hidden size gives up tokens until it fits 100 KB.
+// `beside` a GEMM, above 592 tokens: six tokens and 112 registers.  The GEMM CTA's ten
+// warps of 96 registers are three on one scheduler, and that is what they leave two router
+// warps.  At 128 registers the router waits for the GEMM to end (4096 tokens 696 us per
+// layer against 680 us, 16384 tokens 2249 us against 2178 us); alone the wider tile is the
+// faster one (51 us against 59 us at 4096 tokens, 187 us against 207 us at 16384).
 template <typename IN>
 int32_t launch_router_t(const void *x, const void *wg, const float *bias, const void *wsg, int T,
                         int H, int E, int K, int renorm, int fp32_logits, int32_t *out_idx,
-                        void *out_w, void *out_logits, void *out_shared, cudaStream_t stream) {
+                        void *out_w, void *out_logits, void *out_shared, cudaStream_t stream, bool beside) {
   const int slots = 2 * (sb_device_sm_count() > 0 ? sb_device_sm_count() : 148);
   const size_t row = (size_t)H * sizeof(IN) + (size_t)(E + 1) * sizeof(float), room = 100 * 1024;
   auto launch = launch_router_tile<IN, 1, 2, 4>;
   if (T > slots / 4 && 2 * row <= room) launch = launch_router_tile<IN, 2, 4, 2>;
   if (T > slots && 4 * row <= room) launch = launch_router_tile<IN, 4, 4, 2>;
-  if (T > 2 * slots && 6 * row <= room) launch = launch_router_tile<IN, 6, 4, 2>;
-  if (T > 3 * slots && 6 * row <= room) launch = launch_router_tile<IN, 6, 4, 1>;
+  if (T > 2 * slots && 7 * row <= room) launch = launch_router_tile<IN, 7, 4, 2>;
+  if (T > 7 * slots / 2 && 7 * row <= room) launch = launch_router_tile<IN, 7, 4, 1>;
+  if (beside && T > 2 * slots && 6 * row <= room)
+    launch = T > 3 * slots ? launch_router_tile<IN, 6, 4, 1, 112> : launch_router_tile<IN, 6, 4, 2, 112>;
   return launch(x, wg, bias, wsg, T, H, E, K, renorm, fp32_logits, out_idx, out_w, out_logits, out_shared, stream);
 }
 
@@ -533,7 +535,7 @@ int32_t launch_router_t(const void *x, const void *wg, const float *bias, const 
 
 int32_t launch_router(const void *x, const void *wg, const float *bias, const void *wsg, int T,
                       int H, int E, int K, int renorm, int dtype, int fp32_logits, int32_t *out_idx,
-                      void *out_w, void *out_logits, void *out_shared_scale, cudaStream_t stream) {
+                      void *out_w, void *out_logits, void *out_shared_scale, cudaStream_t stream, bool beside) {
   if (T < 0 || H <= 0 || H % 8 != 0 || E < 1 || E > kMaxExperts || K < 1 || K > kMaxK || K > E)
     return fail(SB_E_INVALID_ARG, "sb_router_topk: need H%%8==0, 1<=K<=8, K<=E<=256 (T=%d H=%d E=%d K=%d)",
                 T, H, E, K);
@@ -547,10 +549,10 @@ int32_t launch_router(const void *x, const void *wg, const float *bias, const vo
     return fail(SB_E_UNSUPPORTED, "sb_router_topk: hidden size %d too large for the token tile", H);
   if (dtype == SB_DTYPE_BF16)
     return launch_router_t<__nv_bfloat16>(x, wg, bias, wsg, T, H, E, K, renorm, fp32_logits, out_idx,
-                                          out_w, out_logits, out_shared_scale, stream);
+                                          out_w, out_logits, out_shared_scale, stream, beside);
   if (dtype == SB_DTYPE_F32)
     return launch_router_t<float>(x, wg, bias, wsg, T, H, E, K, renorm, fp32_logits, out_idx, out_w,
-                                  out_logits, out_shared_scale, stream);
+                                  out_logits, out_shared_scale, stream, beside);
   return fail(SB_E_INVALID_ARG, "sb_router_topk: unknown dtype %d", dtype);
 }
 

@@ -93,7 +93,7 @@ namespace sb {
 int32_t launch_router(const void *x, const void *wg, const float *bias, const void *wsg,
                       int T, int H, int E, int K, int renorm, int dtype, int fp32_logits,
                       int32_t *out_idx, void *out_w, void *out_logits, void *out_shared_scale,
-                      cudaStream_t stream);
+                      cudaStream_t stream, bool beside = false);
 int32_t launch_router_decode(const void *x, const void *wg, const float *bias, const void *wsg, int T, int H,
                              int E, int K, int renorm, int fp32_logits, float *ws, int32_t *out_idx,
                              void *out_w, void *out_logits, void *out_shared_scale, int32_t *expert_offsets,
