@@ -476,7 +476,7 @@ int32_t sb_moe_layer_forward(const sb_moe_layer *L, int32_t *status, void *strea
     rc = launch_decode_experts(L->x, s.item_of_slot, K, s.tile_table, L->slot_of_expert, L->w13, L->w2,
                                s.slot_scale, H, I, L->n_slots, s.hbuf, s.y, Is > 0 ? L->shared_w13 : nullptr,
                                Is > 0 ? L->shared_w2 : nullptr, L->shared_gate_w ? s.shared_scale : nullptr,
-                               Is, T, s.shared_h, s.shared_out, status, 2, 0, nullptr, nullptr, stream, T >= kSharedBesideSortTokens);
+                               Is, T, s.shared_h, s.shared_out, status, 2, 0, nullptr, nullptr, stream);
     if (rc != SB_OK) return rc;
     return launch_combine(s.y, s.slot_of_item, L->topk_idx, Is > 0 ? s.shared_out : nullptr, nullptr, T, H, K,
                           L->out, stream);

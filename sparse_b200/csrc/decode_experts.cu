@@ -114,11 +114,6 @@ __device__ __forceinline__ void reduce_k_slices(float (&acc)[2][4], int warp, in
 // pass 1.  Block task = (group, 8/ks_n x 8 intermediate features); a warp owns
 // 8 features (gate row g in the low half of its MMA rows, up row g in the high
 // half) over one of ks_n slices of H.
-//
-// SHARED_EARLY: the launch before this one is the expert sort, and it let this one
-// start only once the router, and with it whatever made the rows, was complete.  The
-// shared expert's tasks need nothing of the sort and run beside it.
-template <bool SHARED_EARLY>
 __global__ void __launch_bounds__(kThreads, 2)
 decode_gate_up_kernel(const __nv_bfloat16 *__restrict__ x, const int32_t *__restrict__ item_of_slot,
                       int items_per_row, const int32_t *__restrict__ tile_table,
@@ -130,27 +125,19 @@ decode_gate_up_kernel(const __nv_bfloat16 *__restrict__ x, const int32_t *__rest
                       int32_t *__restrict__ status) {
   __shared__ float red[kWarps][8][32];
   pdl_launch_dependents();
-  if (!SHARED_EARLY) pdl_wait();
+  pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, c = lane & 3;
   const int rg_n = kWarps / ks_n, rg = warp / ks_n, ks = warp % ks_n;
   const int feats = rg_n * 8;
-  int n_groups = !SHARED_EARLY && tile_table ? __ldg(tile_table) : 0;
+  const int n_groups = tile_table ? __ldg(tile_table) : 0;
   const int fb_routed = (I + feats - 1) / feats;
   const int fb_shared = shared_w13 ? (I_sh + feats - 1) / feats : 0;
-  long total = (long)n_groups * fb_routed + fb_shared;
-  bool table_ready = !SHARED_EARLY;
+  const long total = (long)n_groups * fb_routed + fb_shared;
   const int chunks = H / 32, per = (chunks + ks_n - 1) / ks_n;
   const int ch0 = min(chunks, ks * per), ch1 = min(chunks, ch0 + per);
-  for (long task_id = blockIdx.x;; task_id += gridDim.x) {
+  for (long task_id = blockIdx.x; task_id < total; task_id += gridDim.x) {
     const bool is_shared = task_id < fb_shared;          // the shared expert's tasks first
-    if (SHARED_EARLY && !is_shared && !table_ready) {
-      pdl_wait();
-      n_groups = tile_table ? __ldg(tile_table) : 0;
-      total += (long)n_groups * fb_routed;
-      table_ready = true;
-    }
-    if (task_id >= total) break;
     int fb, begin, end, inter;
     const __nv_bfloat16 *wbase;
     __nv_bfloat16 *out;
@@ -361,7 +348,7 @@ int32_t launch_decode_experts(const void *x, const int32_t *item_of_slot, int it
                               void *y, const void *shared_w13, const void *shared_w2, const void *shared_scale,
                               int I_sh, int T, void *shared_h, void *shared_out, int32_t *status,
                               int ctas_per_sm, int max_rows, const void *shared_x,
-                              const unsigned long long *row_dst, cudaStream_t stream, bool shared_early) {
+                              const unsigned long long *row_dst, cudaStream_t stream) {
   if (H % 32 != 0 || I % 32 != 0 || I_sh % 32 != 0)
     return fail(SB_E_UNSUPPORTED, "sb_decode_experts: H, I, I_shared must be multiples of 32");
   if (max_rows <= 0) max_rows = kMaxTok;
@@ -393,11 +380,10 @@ int32_t launch_decode_experts(const void *x, const int32_t *item_of_slot, int it
   // large-shared-memory configuration that kernel needs, or the two could not
   // share an SM; alone, the default split leaves more L1 for the token rows.
   const int carveout = ctas_per_sm == 1 ? (int)cudaSharedmemCarveoutMaxShared : (int)cudaSharedmemCarveoutDefault;
-  auto gate_up = shared_early ? decode_gate_up_kernel<true> : decode_gate_up_kernel<false>;
-  SB_CUDA_CHECK(cudaFuncSetAttribute(gate_up, cudaFuncAttributePreferredSharedMemoryCarveout, carveout));
+  SB_CUDA_CHECK(cudaFuncSetAttribute(decode_gate_up_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, carveout));
   SB_CUDA_CHECK(cudaFuncSetAttribute(decode_down_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, carveout));
   SB_CUDA_CHECK(launch_pdl(
-      gate_up, dim3(grid), dim3(kThreads), 0, stream,
+      decode_gate_up_kernel, dim3(grid), dim3(kThreads), 0, stream,
       static_cast<const __nv_bfloat16 *>(x), item_of_slot, items_per_row, tile_table, slot_of_expert,
       static_cast<const __nv_bfloat16 *>(w13), H, I, n_slots, sb_w13_interleaved(),
       static_cast<__nv_bfloat16 *>(hbuf), static_cast<const __nv_bfloat16 *>(shared_x),

@@ -565,11 +565,6 @@ namespace {
 // kernels.
 constexpr int kSmallMaxItems = 16 * kMaxK;
 
-// BESIDE: the launch behind this one works on the shared expert while this one sorts.
-// It may start only after the wait, when the router and all before it are complete, and
-// the chosen experts stay in shared memory from step to step: a round trip to L2 costs
-// twice its idle time while that launch streams weights.
-template <bool BESIDE>
 __global__ void __launch_bounds__(512)
 route_sort_small_kernel(const float *__restrict__ logits, int T, int E, int K, int renorm, int tile_rows,
                         int tile_cap, int32_t *__restrict__ out_idx, __nv_bfloat16 *__restrict__ out_w,
@@ -579,22 +574,19 @@ route_sort_small_kernel(const float *__restrict__ logits, int T, int E, int K, i
   __shared__ float slog[16][kMaxExperts];
   __shared__ int s_exp[kSmallMaxItems];
   __shared__ int s_off[kMaxExperts + 1];
-  __shared__ __nv_bfloat16 s_w[BESIDE ? kSmallMaxItems : 1];
-  if (!BESIDE) pdl_launch_dependents();
+  pdl_launch_dependents();
   pdl_wait();
-  if (BESIDE) pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp < T) {
     for (int e = lane; e < E; e += 32) slog[warp][e] = logits[(size_t)warp * E + e];
     __syncwarp();
-    warp_softmax_topk<__nv_bfloat16>(slog[warp], E, K, renorm, lane, BESIDE ? s_exp + warp * K : out_idx + warp * K,
-                                     BESIDE ? s_w + warp * K : out_w + warp * K);
+    warp_softmax_topk<__nv_bfloat16>(slog[warp], E, K, renorm, lane, out_idx + (size_t)warp * K,
+                                     out_w + (size_t)warp * K);
   }
-  __syncthreads();                       // this CTA's writes are visible to all its threads
+  __syncthreads();                       // this CTA's global writes are visible to all its threads
   const int n = T * K;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const int e = BESIDE ? s_exp[i] : out_idx[i];
-    if (BESIDE) { out_idx[i] = e; out_w[i] = s_w[i]; }
+    const int e = out_idx[i];
     s_exp[i] = (e >= 0 && e < E) ? e : -1;
   }
   __syncthreads();
@@ -611,7 +603,7 @@ route_sort_small_kernel(const float *__restrict__ logits, int T, int E, int K, i
       slot = 0;
       for (int j = 0; j < n; ++j) slot += (s_exp[j] >= 0 && (s_exp[j] < e || (s_exp[j] == e && j < i))) ? 1 : 0;
       item_of_slot[slot] = i;
-      slot_scale[slot] = BESIDE ? s_w[i] : out_w[i];
+      slot_scale[slot] = out_w[i];
     }
     slot_of_item[i] = slot;
   }
@@ -659,8 +651,7 @@ int32_t launch_router_decode(const void *x, const void *wg, const float *bias, c
     if (T > 16 || !expert_offsets || !slot_of_item || !item_of_slot || !slot_scale)
       return fail(SB_E_INVALID_ARG, "router (decode): sort outputs need T <= 16 and all tables");
     const int warps = T > 4 ? 16 : 4;
-    auto sort = T >= kSharedBesideSortTokens ? route_sort_small_kernel<true> : route_sort_small_kernel<false>;
-    SB_CUDA_CHECK(launch_pdl(sort, dim3(1), dim3(warps * 32), 0, stream,
+    SB_CUDA_CHECK(launch_pdl(route_sort_small_kernel, dim3(1), dim3(warps * 32), 0, stream,
                              static_cast<const float *>(ws), T, E, K, renorm, sb_tile_rows(),
                              T * K / SB_TILE_M + E, out_idx, static_cast<__nv_bfloat16 *>(out_w), expert_offsets,
                              slot_of_item, item_of_slot, static_cast<__nv_bfloat16 *>(slot_scale), tile_table));

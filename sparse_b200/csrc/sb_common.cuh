@@ -30,7 +30,10 @@ void reset_launch_count();
 // still draining, once all of that kernel's CTAs have executed
 // pdl_launch_dependents(); pdl_wait() then blocks until the previous kernel has
 // completed and its writes are visible.  Both are no-ops in a plain launch.
-// Rule for kernels using them: no global memory access before pdl_wait().
+// Rule for kernels using them: no load from and no store to global memory before
+// pdl_wait(), also not of data that is older than the previous kernel: what earlier
+// kernels wrote is promised to be visible behind the wait only.  (Asking weights into
+// L2 with a prefetch reads nothing.)
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -77,11 +80,6 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return *reinterpret_cast<uint32_t *>(&v);
 }
 
-// Decode-sized layer pass: from this many tokens the shared expert's gate/up tasks run
-// beside the expert sort (97 against 100 us at 8 tokens, 138 against 147 us at 16;
-// at one token the loaded memory system makes the sort the longer part: 48 against 46.5 us).
-constexpr int kSharedBesideSortTokens = 2;
-
 // Tile table layout shared by sb_permute and the grouped GEMM.
 constexpr int kTileHeaderInts = 4;   // [0] = number of row tiles
 constexpr int kTileEntryInts = 4;    // expert, row_begin, row_end, 0
@@ -120,7 +118,7 @@ int32_t launch_decode_experts(const void *x, const int32_t *item_of_slot, int it
                               void *y, const void *shared_w13, const void *shared_w2,
                               const void *shared_scale, int I_sh, int T, void *shared_h, void *shared_out,
                               int32_t *status, int ctas_per_sm, int max_rows, const void *shared_x,
-                              const unsigned long long *row_dst, cudaStream_t stream, bool shared_early = false);
+                              const unsigned long long *row_dst, cudaStream_t stream);
 int32_t launch_combine(const void *rows_out, const int32_t *slot_of_item, const int32_t *idx,
                        const void *shared_out, const void *shared_scale, int T, int H, int K, void *out,
                        cudaStream_t stream);
