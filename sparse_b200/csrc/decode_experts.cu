@@ -362,16 +362,13 @@ int32_t launch_decode_experts(const void *x, const int32_t *item_of_slot, int it
   if (sms <= 0) return fail(SB_E_CUDA, "sb_decode_experts: no CUDA device");
   const int grid = sms * (ctas_per_sm == 1 ? 1 : 2);       // grid-stride over the block tasks
   // K slices per row group (measured on B200: 2 slices for 64 chunks of 32
-  // elements, 1 for 44, 4 for 176 beat finer splits by up to 8 % at 8 tokens)
+  // elements, 1 for 44, 4 for 176 beat finer splits by up to 8 % at 8 tokens).
+  // From the row lengths alone: the slices set the order of a row's fp32 sum, and a
+  // row has the same bits from the one-GPU layer, the expert-parallel step, the local
+  // expert cache and the offloaded layer's waves, which call this with other counts
+  // of tokens and groups.
   auto slices = [](int k) { const int ch = k / 32; return ch > 128 ? 4 : ch > 48 ? 2 : 1; };
-  const int ks1 = slices(H);
-  int ks2_routed = slices(I), ks2_shared = slices(I_sh > 0 ? I_sh : I);
-  // The down pass of one token has 128 tasks for 296 CTAs, and which SMs the busy ones
-  // land on is chance: twice the K slices, twice the tasks (751 -> 734 us per step of
-  // nine DeepSeek-shaped layers at one token).
-  const long down_tasks = (tile_table ? (long)T * items_per_row : 0) * ((H * ks2_routed + 127) / 128) +
-                          (shared_w13 ? (H * ks2_shared + 127) / 128 : 0);
-  if (2 * down_tasks <= grid) { ks2_routed *= 2; ks2_shared = ks2_shared < 8 ? ks2_shared * 2 : 8; }
+  const int ks1 = slices(H), ks2_routed = slices(I), ks2_shared = slices(I_sh > 0 ? I_sh : I);
   // (Splitting K finer at one or two tokens, so that the 352 pass-1 / 128 pass-2
   // tasks of a single token spread over all CTAs in several small rounds, was
   // measured slower on B200: 50 us against 45 us per layer at one token.  The

@@ -2,7 +2,8 @@
 import pytest
 import torch
 
-from sparse_b200 import synth
+from sparse_b200 import ops, synth
+from sparse_b200._lib import lib, check
 from sparse_b200.layer import LayerRunner
 from sparse_b200.model import random_layer_weights
 
@@ -43,3 +44,67 @@ def test_rows_written_just_before_a_pass_are_the_ones_it_reads(t):
     for i, o in enumerate(out):
         assert torch.equal(o, want[i % 3])
     runner.check_status()
+
+
+@pytest.mark.parametrize("t", [1, 2, 3, 4, 5, 16])
+def test_decode_rows_do_not_depend_on_how_the_experts_are_called(t):
+    """The Qwen shape's rows through the one-GPU layer, and through the calls that the
+    expert-parallel step, the local expert cache and the offloaded layer make: the same bits."""
+    shape, w = synth.QWEN_MOE, _weights("QWEN_MOE")
+    h, i, e, k = shape.hidden, shape.inter, shape.num_experts, shape.top_k
+    runner = LayerRunner(w, k, t)
+    x = _rows(t, h, 70 + t)
+    want, idx, wts, _ = runner.forward(x)
+    gate = ops.router_topk(x, w.router_w, k, bias=w.router_bias, w_shared_gate=w.shared_gate_w)[3]
+    p = ops.permute(x, idx.reshape(-1), e, k, item_scale=wts.reshape(-1))
+    hbuf = torch.empty((p.r_cap, i), dtype=BF, device=DEV)
+    status = torch.zeros((1,), dtype=torch.int32, device=DEV)
+    stream = torch.cuda.current_stream(DEV).cuda_stream
+    shared_h = torch.empty((t, shape.shared_inter), dtype=BF, device=DEV)
+
+    def experts(y, slots, shared_out):
+        on = shared_out is not None
+        check(lib.sb_decode_experts(
+            x.data_ptr(), p.item_of_slot.data_ptr(), k, p.tile_table.data_ptr(), slots.data_ptr(), w.w13.data_ptr(),
+            w.w2.data_ptr(), p.slot_scale.data_ptr(), h, i, w.n_slots, hbuf.data_ptr(), y.data_ptr(),
+            w.shared_w13.data_ptr() if on else None, w.shared_w2.data_ptr() if on else None,
+            gate.data_ptr() if on else None, shape.shared_inter if on else 0, t,
+            shared_h.data_ptr() if on else None, shared_out.data_ptr() if on else None, status.data_ptr(), stream),
+            "sb_decode_experts")
+
+    def mixed(y, dst):
+        check(lib.sb_grouped_swiglu_mixed(
+            p.rows.data_ptr(), p.tile_table.data_ptr(), w.w13.data_ptr(), w.w2.data_ptr(), w.slot_of_expert.data_ptr(),
+            p.slot_scale.data_ptr(), p.r_cap, h, i, w.n_slots, hbuf.data_ptr(), y.data_ptr(), 0, None, None, None,
+            None, 0, 0, None, None, dst.data_ptr() if dst is not None else None, status.data_ptr(), stream),
+            "sb_grouped_swiglu_mixed")
+
+    # the shared expert by itself, as the expert-parallel step calls it
+    alone = torch.empty((t, h), dtype=BF, device=DEV)
+    check(lib.sb_decode_experts(
+        x.data_ptr(), None, 1, None, None, None, None, None, h, i, 1, None, None, w.shared_w13.data_ptr(),
+        w.shared_w2.data_ptr(), gate.data_ptr(), shape.shared_inter, t, shared_h.data_ptr(), alone.data_ptr(),
+        status.data_ptr(), stream), "sb_decode_experts(shared)")
+    got = {}
+    y = {name: torch.full((p.r_cap, h), float("nan"), dtype=BF, device=DEV)
+         for name in ("waves", "received", "scattered", "cached")}
+    beside = torch.empty((t, h), dtype=BF, device=DEV)
+    # the offloaded layer: the experts in two launches, the shared one in the first of them
+    even = torch.arange(e, device=DEV) % 2 == 0
+    skip = torch.full_like(w.slot_of_expert, -2)
+    experts(y["waves"], torch.where(even, w.slot_of_expert, skip), beside)
+    experts(y["waves"], torch.where(even, skip, w.slot_of_expert), None)
+    mixed(y["received"], None)
+    row_dst = {name: y[name].data_ptr() + 2 * h * torch.arange(p.r_cap, dtype=torch.int64, device=DEV)
+               for name in ("scattered", "cached")}
+    mixed(y["scattered"], row_dst["scattered"])
+    check(lib.sb_decode_experts_to(
+        x.data_ptr(), p.item_of_slot.data_ptr(), k, p.tile_table.data_ptr(), w.slot_of_expert.data_ptr(),
+        w.w13.data_ptr(), w.w2.data_ptr(), p.slot_scale.data_ptr(), h, i, w.n_slots, hbuf.data_ptr(),
+        row_dst["cached"].data_ptr(), t, status.data_ptr(), stream), "sb_decode_experts_to")
+    got["waves"] = ops.combine(y["waves"], p.slot_of_item, idx, beside, t)
+    for name in ("received", "scattered", "cached"):
+        got[name] = ops.combine(y[name], p.slot_of_item, idx, alone, t)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    assert {name: torch.equal(o, want) for name, o in got.items()} == dict.fromkeys(got, True)
