@@ -45,6 +45,7 @@ class B200MoeBlock:
         # (see `forward_device`); off by default because a graph pins its buffers.
         self.use_graphs = use_graphs
         self._graphs = {}
+        self._graph_reserve = self.runner.reserves
 
     @classmethod
     def from_block_weights(cls, w, device: torch.device, ep_rank: int = 0, ep_size: int = 1,
@@ -109,6 +110,11 @@ class B200MoeBlock:
         return res
 
     def _forward_graphed_local(self, x: torch.Tensor, out: Optional[torch.Tensor], first_row: int = 0) -> torch.Tensor:
+        if self._graph_reserve != self.runner.reserves:
+            # A larger batch has replaced the runner's buffers, which the recorded passes write to.
+            torch.cuda.synchronize(self.device)
+            self._graphs.clear()
+            self._graph_reserve = self.runner.reserves
         dst = self.runner.out[first_row:first_row + x.shape[0]] if out is None else out
         key = (x.data_ptr(), x.shape[0], dst.data_ptr(), first_row)
         ent = self._graphs.get(key)

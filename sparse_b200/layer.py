@@ -120,6 +120,7 @@ class LayerRunner:
         self.top_k, self.renorm, self.fp32_logits = top_k, renorm, fp32_logits
         self.want_logits = want_logits
         self.max_tokens = 0
+        self.reserves = 0            # counts the times the buffers below were replaced
         self.status = torch.zeros((1,), dtype=torch.int32, device=weights.device)
         dev_index = weights.device.index if weights.device.index is not None else torch.cuda.current_device()
         _lib.init_device(dev_index)
@@ -129,6 +130,7 @@ class LayerRunner:
         w, dev = self.w, self.w.device
         tokens = max(int(tokens), 1)
         self.max_tokens = tokens
+        self.reserves += 1
         nbytes = lib.sb_moe_layer_workspace_bytes(tokens, w.hidden, w.num_experts, self.top_k,
                                                   w.inter, w.shared_inter)
         # over-allocate so the base can be rounded up to 1024 bytes

@@ -4,6 +4,7 @@ import torch
 
 from sparse_b200 import ops, synth
 from sparse_b200._lib import lib, check
+from sparse_b200.block import B200MoeBlock
 from sparse_b200.layer import LayerRunner
 from sparse_b200.model import random_layer_weights
 
@@ -108,3 +109,25 @@ def test_decode_rows_do_not_depend_on_how_the_experts_are_called(t):
     torch.cuda.synchronize()
     assert int(status.item()) == 0
     assert {name: torch.equal(o, want) for name, o in got.items()} == dict.fromkeys(got, True)
+
+
+def test_recorded_passes_end_with_the_buffers_they_write_to():
+    """A pass is recorded, a batch above `max_tokens` replaces the scratch and the result
+    buffers, the first buffers come again: their pass writes to the new ones."""
+    shape, w = synth.TINY, _weights("TINY")
+    block = B200MoeBlock(w, shape.top_k, 64, use_graphs=True)
+    plain = B200MoeBlock(w, shape.top_k, 200)
+    x, out = _rows(48, shape.hidden, 1), torch.empty((48, shape.hidden), dtype=BF, device=DEV)
+    for seed in (2, 3, 4):
+        x.copy_(_rows(48, shape.hidden, seed))
+        block.forward_device(x, out)
+    assert len(block._graphs) == 1
+    big = _rows(200, shape.hidden, 5)
+    assert torch.equal(block.forward_device(big), plain.forward_device(big))
+    for seed in (6, 7):
+        x.copy_(_rows(48, shape.hidden, seed))
+        block.forward_device(x, out)
+        assert torch.equal(out, plain.forward_device(x))
+        for a, b in zip((*block.topk(48), block.router_logits(48)), (*plain.topk(48), plain.router_logits(48))):
+            assert torch.equal(a, b)
+    block.check_status()
