@@ -129,6 +129,12 @@ class LayerRunner:
     def _reserve(self, tokens: int) -> None:
         w, dev = self.w, self.w.device
         tokens = max(int(tokens), 1)
+        if self.reserves:
+            # passes of the current stream may still be at work in the buffers to be replaced
+            stream = torch.cuda.current_stream(dev)
+            for old in (self._ws_raw, self.out, self.topk_idx, self.topk_w, self.logits):
+                if old is not None:
+                    old.record_stream(stream)
         self.max_tokens = tokens
         self.reserves += 1
         nbytes = lib.sb_moe_layer_workspace_bytes(tokens, w.hidden, w.num_experts, self.top_k,

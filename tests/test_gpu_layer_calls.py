@@ -131,3 +131,27 @@ def test_recorded_passes_end_with_the_buffers_they_write_to():
         for a, b in zip((*block.topk(48), block.router_logits(48)), (*plain.topk(48), plain.router_logits(48))):
             assert torch.equal(a, b)
     block.check_status()
+
+
+def test_replaced_scratch_is_not_given_away_while_a_pass_uses_it():
+    """Passes wait in a stream of their own; the scratch that a larger batch replaces must not
+    serve another stream's tensor before they are through."""
+    shape = synth.TINY
+    runner = LayerRunner(_weights("TINY"), shape.top_k, 64)
+    small, big = _rows(64, shape.hidden, 1), _rows(300, shape.hidden, 2)
+    stream = torch.cuda.Stream(device=DEV)
+    with torch.cuda.stream(stream):                       # kernels loaded, the stream's memory at hand
+        first = LayerRunner(_weights("TINY"), shape.top_k, 300)
+        first.forward(small), first.forward(big)
+        del first
+        torch.cuda._sleep(1)
+    torch.full((8,), 255, dtype=torch.uint8, device=DEV)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(400_000_000)                    # some 200 ms of the stream
+        runner.forward(small)
+        sizes = [runner._ws_raw.numel(), runner.out.numel() * 2]
+        runner.forward(big)
+    others = [torch.full((n,), 255, dtype=torch.uint8, device=DEV) for n in sizes for _ in range(4)]
+    torch.cuda.synchronize()
+    assert all(bool((o == 255).all()) for o in others)
