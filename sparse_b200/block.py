@@ -144,7 +144,7 @@ class B200MoeBlock:
                                         device=self.device)
         xd = self._x_stage[:t]
         stream = torch.cuda.current_stream(self.device)
-        parts = self._host_parts(t)
+        parts = self._host_parts(x_host, out_host)
         if parts == 1:
             xd.copy_(x_host, non_blocking=True)
             out = self.forward_device(xd)
@@ -160,29 +160,41 @@ class B200MoeBlock:
         launches = 0
         rows = [t * i // parts // 16 * 16 for i in range(parts)] + [t]
         arrived = []
-        with torch.cuda.stream(inward):
-            for r0, r1 in zip(rows, rows[1:]):
-                xd[r0:r1].copy_(x_host[r0:r1], non_blocking=True)
-                arrived.append(inward.record_event())
-        for r0, r1, there in zip(rows, rows[1:], arrived):
-            stream.wait_event(there)
-            out = self._forward_local(xd[r0:r1], None, r0)
-            launches += self.last_launches
-            outward.wait_stream(stream)
-            with torch.cuda.stream(outward):
-                out_host[r0:r1].copy_(out, non_blocking=True)
+        try:
+            with torch.cuda.stream(inward):
+                for r0, r1 in zip(rows, rows[1:]):
+                    xd[r0:r1].copy_(x_host[r0:r1], non_blocking=True)
+                    arrived.append(inward.record_event())
+            for r0, r1, there in zip(rows, rows[1:], arrived):
+                stream.wait_event(there)
+                out = self._forward_local(xd[r0:r1], None, r0)
+                launches += self.last_launches
+                outward.wait_stream(stream)
+                with torch.cuda.stream(outward):
+                    out_host[r0:r1].copy_(out, non_blocking=True)
+        finally:                                  # also when a part is refused: no copy outlives the call
+            stream.wait_stream(inward)
+            stream.wait_stream(outward)
+            stream.synchronize()
         self.last_launches = launches
-        stream.wait_stream(outward)
-        stream.synchronize()
 
     _copy_lanes = None
 
-    def _host_parts(self, tokens: int) -> int:
+    def _host_parts(self, x_host: torch.Tensor, out_host: torch.Tensor) -> int:
         """Parts a host batch is passed in.  Splitting hides all copies but the first
         part's in and the last part's out (75 ns a row each way), and costs the layer
         time that two half batches take longer than one: from 3072 rows the copies
-        win (a batch below streams the expert weights twice for little)."""
+        win (a batch below streams the expert weights twice for little).  A result that
+        is not row for row the input's counterpart, or that lies over other rows of
+        it, is copied as a whole."""
+        tokens = x_host.shape[0]
         if self._ep is not None or tokens < 3072 or tokens > self.runner.max_tokens:
+            return 1
+        if out_host.shape != x_host.shape:
+            return 1
+        if out_host.untyped_storage().data_ptr() == x_host.untyped_storage().data_ptr() and (
+                out_host.data_ptr() != x_host.data_ptr() or out_host.stride() != x_host.stride()
+                or out_host.dtype != x_host.dtype):
             return 1
         return max(2, tokens // 4096)
 
