@@ -42,7 +42,27 @@ def test_host_batches_equal_device_batches(weights, t, graphs):
         assert torch.equal(out, want.cpu())
         for a, b in zip((*block.topk(t), block.router_logits(t)), (*other.topk(t), other.router_logits(t))):
             assert torch.equal(a, b)
+        if call == 0:                         # the first pass on new buffers records nothing
+            assert not block._graphs and not any(block._part_graphs.values())
     block.check_status()
+
+
+def test_a_recorded_part_takes_no_place_of_a_recorded_batch(weights):
+    """Split batches of many sizes leave the graphs of a serving loop's own buffers alone."""
+    t = 4096
+    block = B200MoeBlock(weights, SHAPE.top_k, t, use_graphs=True)
+    x = _rows(64, 1).to(DEV)
+    y = torch.empty_like(x)
+    block.forward_device(x, y)
+    block.forward_device(x, y)
+    kept = dict(block._graphs)
+    assert len(kept) == 1
+    for n in range(3072, 3072 + 20):
+        rows, out = _rows(n, n), _pinned(n, SHAPE.hidden)
+        for _ in range(2):
+            block.forward_host(rows.pin_memory(), out)
+        assert torch.equal(out, block.runner.forward(rows.to(DEV))[0].cpu())
+    assert all(block._graphs.get(k) is v for k, v in kept.items())
 
 
 @pytest.mark.parametrize("t", [2048, 3072])
