@@ -358,6 +358,10 @@ int32_t launch_decode_experts(const void *x, const int32_t *item_of_slot, int it
     return fail(SB_E_INVALID_ARG, "sb_decode_experts: null pointer");
   if ((shared_w13 != nullptr) != (shared_w2 != nullptr) || (shared_w13 && (!shared_h || !shared_out)))
     return fail(SB_E_INVALID_ARG, "sb_decode_experts: shared expert arguments go together");
+  const auto whole = [](const void *p) { return aligned(p, 16); };        // the kernels read 16 bytes at a time
+  if ((tile_table && !(whole(tile_table) && whole(x) && whole(w13) && whole(w2) && whole(hbuf))) ||
+      (shared_w13 && !(whole(shared_x) && whole(shared_w13) && whole(shared_w2) && whole(shared_h))))
+    return fail(SB_E_INVALID_ARG, "sb_decode_experts: rows, weights, tables and intermediate rows must be 16-byte aligned");
   const int sms = sb_device_sm_count();
   if (sms <= 0) return fail(SB_E_CUDA, "sb_decode_experts: no CUDA device");
   const int grid = sms * (ctas_per_sm == 1 ? 1 : 2);       // grid-stride over the block tasks

@@ -662,6 +662,8 @@ int32_t sb_attn_decode(const void *q, int32_t q_stride, const void *cache_k, con
     return fail(SB_E_INVALID_ARG, "sb_attn_decode: bad shape");
   if (B == 0) return SB_OK;
   if (!q || !cache_k || !cache_v || !seq_lens || !ws || !out) return fail(SB_E_INVALID_ARG, "sb_attn_decode: null pointer");
+  if (!aligned(cache_k, 4) || !aligned(cache_v, 4) || !aligned(ws, 4))
+    return fail(SB_E_INVALID_ARG, "sb_attn_decode: cache_k, cache_v, ws must be 4-byte aligned");
   if (ws_bytes < sb_attn_decode_workspace_bytes(B, n_q, dv, n_split))
     return fail(SB_E_WORKSPACE, "sb_attn_decode: workspace too small");
   cudaStream_t st = static_cast<cudaStream_t>(stream);

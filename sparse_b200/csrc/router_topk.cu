@@ -639,6 +639,8 @@ int32_t launch_router_decode(const void *x, const void *wg, const float *bias, c
   if (T <= 0) return SB_OK;
   if (H % 8 != 0 || E < 1 || E > kMaxExperts || K < 1 || K > kMaxK || K > E || !ws)
     return fail(SB_E_INVALID_ARG, "router (decode): bad arguments");
+  if (!aligned(x, 16) || !aligned(wg, 16) || (wsg && !aligned(wsg, 16)))
+    return fail(SB_E_INVALID_ARG, "router (decode): x, wg, w_shared_gate must be 16-byte aligned");
   const int NR = E + (wsg ? 1 : 0);
   dim3 grid(T, (NR + kRouterWarps - 1) / kRouterWarps);
   SB_CUDA_CHECK(launch_pdl(router_rows_kernel<__nv_bfloat16>, grid, dim3(kRouterThreads), 0, stream,

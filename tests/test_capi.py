@@ -60,6 +60,29 @@ def test_bad_arguments_are_rejected_with_a_message():
     assert lib.sb_combine(None, None, None, None, 0, 2048, 4, None, None) == 0
 
 
+def test_operands_off_their_load_width_are_refused():
+    """The decode kernels read 16 bytes at a time (the caches 4): an address off that is an
+    argument error, not a fault.  (The addresses are never read: the checks come first.)"""
+    from sparse_b200._lib import lib
+    ok = 1 << 20
+
+    def experts(**off):
+        a = dict.fromkeys(("x", "table", "w13", "w2", "hbuf", "y", "s13", "s2", "sh", "so"), ok)
+        a.update({k: ok + v for k, v in off.items()})
+        return lib.sb_decode_experts(a["x"], None, 1, a["table"], None, a["w13"], a["w2"], None, 64, 64, 1, a["hbuf"],
+                                     a["y"], a["s13"], a["s2"], None, 64, 1, a["sh"], a["so"], None, None)
+
+    for name in ("x", "table", "w13", "w2", "hbuf", "s13", "s2", "sh"):
+        assert experts(**{name: 8}) == -1 and b"aligned" in lib.sb_last_error_string(), name
+    for x, w, g in ((2, 0, 0), (0, 8, 0), (0, 0, 4)):
+        rc = lib.sb_route_decode(ok + x, ok + w, None, ok + g, 1, 64, 8, 2, 0, 0, ok, ok, ok, None, ok, ok, ok, ok, ok, ok,
+                                 None)
+        assert rc == -1 and b"aligned" in lib.sb_last_error_string()
+    for k, v in ((2, 0), (0, 2)):
+        rc = lib.sb_attn_decode(ok, 0, ok + k, ok + v, ok, 1, 1, 1, 128, 128, 16, 1.0, 1, ok, 1 << 20, ok, None)
+        assert rc == -1 and b"aligned" in lib.sb_last_error_string()
+
+
 def test_struct_layout_matches_header():
     from sparse_b200._lib import MoeLayer, lib
     assert C.sizeof(MoeLayer) == lib.sb_moe_layer_struct_bytes()
