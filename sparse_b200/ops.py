@@ -121,15 +121,22 @@ def grouped_swiglu(rows: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor,
 
 
 def dense_swiglu(rows: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor) -> torch.Tensor:
-    """One SwiGLU FFN over all rows: rows [T,H]; w13 [1,2I,H]; w2 [1,H,I] -> [T,H].
+    """One SwiGLU FFN over all rows: rows [T,H]; w13 [1,2I,H]; w2 [1,H,I] -> [T,H], bf16.
 
     Up to `_lib.DECODE_MAX_TOKENS` rows the FFN is its weights' bytes, and the streaming
     kernels read them with every SM; the tile kernel would walk the output in 256-row
     tiles, for 10944 x 2048 eight of them in the down pass, on eight of the 74 CTA pairs
-    (26 + 52 us for 134 MB at one row)."""
+    (26 + 52 us for 134 MB at one row).  Operands are those of the tile kernel either way."""
     t, h = rows.shape
     i = w13.shape[1] // 2
-    if t > _lib.DECODE_MAX_TOKENS or h % 64 != 0 or i % 64 != 0:
+    if w13.shape[1:] != (2 * i, h) or w2.shape[1:] != (h, i):
+        raise RuntimeError("dense_swiglu: rows %s, w13 %s and w2 %s do not fit" % (
+            tuple(rows.shape), tuple(w13.shape), tuple(w2.shape)))
+    for v in (rows, w13, w2):
+        if v.dtype != torch.bfloat16 or v.device != rows.device:
+            raise RuntimeError("dense_swiglu needs bf16 operands on one device")
+    if t > _lib.DECODE_MAX_TOKENS or h % 64 != 0 or i % 64 != 0 or any(
+            _ptr(v) % 128 != 0 for v in (rows, w13, w2)):
         return grouped_swiglu(rows, w13, w2, dense_rows=t)[0][:t]
     hbuf = torch.empty((t, i), dtype=torch.bfloat16, device=rows.device)
     out = torch.empty((t, h), dtype=torch.bfloat16, device=rows.device)
@@ -140,13 +147,31 @@ def dense_swiglu(rows: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor) -> tor
     return out
 
 
+def _streams(rows: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor]) -> bool:
+    """Whether `sb_decode_linear` takes the operands: a few packed bf16 rows, whole 16-byte
+    vectors, nothing that wants a gradient."""
+    if rows.dim() != 2 or weight.dim() != 2 or not 0 < rows.shape[0] <= _lib.DECODE_MAX_TOKENS:
+        return False
+    n, k = weight.shape
+    if n == 0 or k == 0 or k % 32 != 0 or rows.shape[1] != k or (bias is not None and bias.shape != (n,)):
+        return False
+    operands = [v for v in (rows, weight, bias) if v is not None]
+    if any(v.dtype != torch.bfloat16 or not v.is_cuda or v.device != rows.device or not v.is_contiguous()
+           for v in operands):
+        return False
+    if torch.is_grad_enabled() and any(v.requires_grad for v in operands):
+        return False
+    return rows.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
+
+
 def linear(rows: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """rows [T,K] . weight [N,K]^T (+ bias): the weight-streaming kernel up to
-    `_lib.DECODE_MAX_TOKENS` rows (8 MB of weights: 7 us through the library at one
-    to eight rows, most of them not spent on the bytes), the library's GEMM above."""
-    (t, k), n = rows.shape, weight.shape[0]
-    if t > _lib.DECODE_MAX_TOKENS or k % 32 != 0 or not rows.is_contiguous():
+    `_lib.DECODE_MAX_TOKENS` bf16 rows (8 MB of weights: 7 us through the library at one
+    to eight rows, most of them not spent on the bytes), the library's GEMM above and
+    for all operands that the kernel is not made for."""
+    if not _streams(rows, weight, bias):
         return torch.nn.functional.linear(rows, weight, bias)
+    (t, k), n = rows.shape, weight.shape[0]
     out = torch.empty((t, n), dtype=torch.bfloat16, device=rows.device)
     with torch.cuda.device(rows.device):
         check(lib.sb_decode_linear(_ptr(rows), _ptr(weight), _ptr(bias), t, n, k, _ptr(out), _stream(rows)),
