@@ -385,15 +385,17 @@ attn_decode_kernel(const __nv_bfloat16 *__restrict__ q, int q_stride, const __nv
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (ok[u]) m_new = fmaxf(m_new, s[u]);
-    // a group that has seen no key yet (or only scores of -inf) keeps its zero sums
-    const float corr = m == m_new ? 1.f : __expf(m - m_new);
+    // a group that has seen no key yet, or only scores of -inf, keeps its zero sums: those
+    // keys have the weight exp(-inf - 0) = 0
+    const float m_ref = m_new == -INFINITY ? 0.f : m_new;
+    const float corr = m == m_new ? 1.f : __expf(m - m_ref);
     l *= corr;
 #pragma unroll
     for (int e = 0; e < NV * 8; ++e) acc[e] *= corr;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (!ok[u]) continue;                   // a masked key adds nothing, whatever its clamped row holds
-      const float p = __expf(s[u] - m_new);
+      const float p = __expf(s[u] - m_ref);
       l += p;
 #pragma unroll
       for (int n = 0; n < NV; ++n) {
@@ -411,7 +413,7 @@ attn_decode_kernel(const __nv_bfloat16 *__restrict__ q, int q_stride, const __nv
 #pragma unroll
   for (int off = kAttnLanes; off <= 16; off <<= 1) {
     const float mm = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
-    const float c = m == -INFINITY ? 0.f : __expf(m - mm);      // (only scores of -inf: l is NaN, and NaN * 0 stays NaN)
+    const float c = m == -INFINITY ? 0.f : __expf(m - mm);
     l *= c;
     l += __shfl_xor_sync(0xffffffffu, l, off);
 #pragma unroll

@@ -172,3 +172,34 @@ def test_linear_on_either_side_of_the_streaming_limit(t, n, k, with_bias):
     # fp32 sums of at most 2048 products of order 1 / sqrt(k), one rounding to bf16
     assert got.shape == (t, n)
     assert float(((got.double() - want).abs() - 2.0 ** -8 * want.abs()).max()) < 1e-4
+
+
+@pytest.mark.parametrize("n_q,n_kv,dk,dv", [(2, 2, 128, 128), (2, 1, 192, 128), (2, 2, 64, 64)])
+@pytest.mark.parametrize("n_split", [1, 4])
+def test_attn_decode_scores_of_minus_infinity_weigh_nothing(n_q, n_kv, dk, dv, n_split):
+    """Keys with a score of -inf alone in a group's first turn, in a warp, in a split; a
+    sequence of nothing else gives zeros, as an empty one does."""
+    torch.manual_seed(dk + n_split)
+    lens = [5, 17, 40, 97, 33, 6]
+    dead = [[0], [16], [0, 1, 2, 3, 20], [0, 31, 32, 96], list(range(0, 33, 2)), list(range(6))]
+    b, s_max = len(lens), max(lens)
+    q = (torch.rand(b, n_q, dk, device=DEV) + 0.1).to(BF)
+    ck = torch.randn(b, s_max, n_kv, dk, device=DEV).to(BF)
+    cv = torch.randn(b, s_max, n_kv, dv, device=DEV).to(BF)
+    for i, keys in enumerate(dead):
+        ck[i, keys, :, 3] = float("-inf")
+    seq_lens = torch.tensor(lens, dtype=torch.int32, device=DEV)
+    ws = torch.empty(lib.sb_attn_decode_workspace_bytes(b, n_q, dv, n_split), dtype=torch.uint8, device=DEV)
+    out = torch.empty(b, n_q, dv, dtype=BF, device=DEV)
+    check(lib.sb_attn_decode(q.data_ptr(), 0, ck.data_ptr(), cv.data_ptr(), seq_lens.data_ptr(), b, n_q, n_kv, dk, dv,
+                             s_max, 1.0 / math.sqrt(dk), n_split, ws.data_ptr(), ws.numel(), out.data_ptr(), _stream()),
+          "sb_attn_decode")
+    torch.cuda.synchronize()
+    assert float(out[5].abs().max()) == 0.0
+    for i, n in enumerate(lens[:5]):
+        kk = ck[i, :n].float().repeat_interleave(n_q // n_kv, dim=1)
+        vv = cv[i, :n].float().repeat_interleave(n_q // n_kv, dim=1)
+        p = torch.softmax(torch.einsum("hd,nhd->hn", q[i].float(), kk) / math.sqrt(dk), dim=-1)
+        want = torch.einsum("hn,nhd->hd", p, vv)
+        # fp32 sums, one rounding to bf16: half a step of 2^-8 of a value, and __expf's 2^-21
+        assert float(((out[i].float() - want).abs() - 2.0 ** -8 * want.abs()).max()) < 1e-4
