@@ -19,6 +19,7 @@ namespace sb {
 namespace {
 
 constexpr int kNormThreads = 256;
+constexpr int kMaxNormRow = 16384;    // eight 16-byte vectors a thread
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
@@ -157,6 +158,9 @@ int32_t launch_add_rmsnorm(void *residual, int res_stride, const void *delta, co
                         : nv <= 4 ? add_rmsnorm_vec_kernel<4> : add_rmsnorm_vec_kernel<8>;
     SB_CUDA_CHECK(launch_pdl(kern, dim3(T), dim3(kNormThreads), 0, stream, res, (size_t)res_stride, d1, d2, ww, eps, H, oo));
   } else {
+    if ((size_t)H * sizeof(float) > 47 * 1024)          // (with the partial sums more than the 48 KB of any launch)
+      SB_CUDA_CHECK(cudaFuncSetAttribute(add_rmsnorm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         kMaxNormRow * (int)sizeof(float)));
     add_rmsnorm_kernel<<<T, kNormThreads, (size_t)H * sizeof(float), stream>>>(res, (size_t)res_stride, d1, d2, ww, eps,
                                                                                H, oo);
   }
@@ -579,7 +583,7 @@ extern "C" {
 
 int32_t sb_add_rmsnorm(void *residual, const void *delta, const void *delta2, const void *weight, float eps,
                        int32_t T, int32_t H, void *out, void *stream) {
-  if (T < 0 || H <= 0 || H > 16384) return fail(SB_E_INVALID_ARG, "sb_add_rmsnorm: bad shape (T=%d H=%d)", T, H);
+  if (T < 0 || H <= 0 || H > kMaxNormRow) return fail(SB_E_INVALID_ARG, "sb_add_rmsnorm: bad shape (T=%d H=%d)", T, H);
   if (T == 0) return SB_OK;
   if (!residual || (!out && !delta) || (out && !weight) || (delta2 && !delta))
     return fail(SB_E_INVALID_ARG, "sb_add_rmsnorm: null pointer");
@@ -588,7 +592,7 @@ int32_t sb_add_rmsnorm(void *residual, const void *delta, const void *delta2, co
 
 int32_t sb_rmsnorm_rows(const void *rows, int32_t row_stride, const void *weight, float eps, int32_t T, int32_t H,
                         void *out, void *stream) {
-  if (T < 0 || H <= 0 || H > 16384 || row_stride < H)
+  if (T < 0 || H <= 0 || H > kMaxNormRow || row_stride < H)
     return fail(SB_E_INVALID_ARG, "sb_rmsnorm_rows: bad shape (T=%d H=%d stride=%d)", T, H, row_stride);
   if (T == 0) return SB_OK;
   if (!rows || !weight || !out) return fail(SB_E_INVALID_ARG, "sb_rmsnorm_rows: null pointer");

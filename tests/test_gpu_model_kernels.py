@@ -57,8 +57,6 @@ def test_rmsnorm_vectors_give_the_bits_of_single_elements(t, h, with_delta):
     w = torch.randn(h, device=DEV).to(BF)
     got = []
     for off in (0, 1):
-        if off and h > 12288:                         # (the element kernel's row must fit 48 KB as floats)
-            continue
         r, d, o = _shifted(resid, off), _shifted(delta, off), _shifted(resid, off)
         check(lib.sb_add_rmsnorm(r.data_ptr(), d.data_ptr() if with_delta else None, None, w.data_ptr(), 1e-6, t, h,
                                  o.data_ptr(), _stream()), "sb_add_rmsnorm")
@@ -203,3 +201,19 @@ def test_attn_decode_scores_of_minus_infinity_weigh_nothing(n_q, n_kv, dk, dv, n
         want = torch.einsum("hn,nhd->hd", p, vv)
         # fp32 sums, one rounding to bf16: half a step of 2^-8 of a value, and __expf's 2^-21
         assert float(((out[i].float() - want).abs() - 2.0 ** -8 * want.abs()).max()) < 1e-4
+
+
+@pytest.mark.parametrize("h", [12288, 12296, 16384])
+def test_wide_rows_off_a_vector_boundary(h):
+    """Rows whose fp32 copy is larger than 48 KB, on addresses that are no whole vectors."""
+    torch.manual_seed(h)
+    rows, w = torch.randn(2, h, device=DEV).to(BF), torch.randn(h, device=DEV).to(BF)
+    got = []
+    for off in (0, 1):
+        r, o = _shifted(rows, off), _shifted(rows, off)
+        check(lib.sb_rmsnorm_rows(r.data_ptr(), h, w.data_ptr(), 1e-6, 2, h, o.data_ptr(), _stream()), "sb_rmsnorm_rows")
+        check(lib.sb_add_rmsnorm(r.data_ptr(), rows.data_ptr(), None, w.data_ptr(), 1e-6, 2, h, o.data_ptr(), _stream()),
+              "sb_add_rmsnorm")
+        got.append((r, o))
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(*got))
