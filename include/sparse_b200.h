@@ -575,7 +575,7 @@ int32_t sb_moe_layer_forward(const sb_moe_layer *layer, int32_t *status, void *s
  *                  (0 = densely packed), so q, k, v may be column slices of
  *                  one fused projection output.
  * sb_decode_linear out [T,N] = bf16(x [T,K] . w [N,K]^T + bias [N] (may be NULL)) for
- *                  T <= SB_DECODE_MAX_TOKENS, fp32 sums, K a multiple of 32.
+ *                  T <= SB_DECODE_MAX_TOKENS, fp32 sums, K a multiple of 32, N <= 2^27.
  * sb_rmsnorm_rows  out [T,H] = weight * bf16(row * rsqrt(mean(row^2) + eps)) of rows
  *                  that lie `row_stride` elements apart (column slices of a
  *                  projection output); the rows themselves are not written.
@@ -593,7 +593,7 @@ int32_t sb_moe_layer_forward(const sb_moe_layer *layer, int32_t *status, void *s
  *                  sb_attn_decode_workspace_bytes.  Built for (dk,dv) =
  *                  (128,128), (192,128), (64,64).
  * sb_argmax_rows   out[b] = index of the largest of the V logits of row b, the first
- *                  one among equals, NaN above every number.
+ *                  one among equals, NaN above every number; V <= 2^30.
  */
 int32_t sb_add_rmsnorm(void *residual, const void *delta, const void *delta2, const void *weight, float eps,
                        int32_t T, int32_t H, void *out, void *stream);

@@ -407,8 +407,8 @@ int32_t launch_decode_experts(const void *x, const int32_t *item_of_slot, int it
 extern "C" int32_t sb_decode_linear(const void *x, const void *w, const void *bias, int32_t T, int32_t N, int32_t K,
                                     void *out, void *stream) {
   using namespace sb;
-  if (T < 0 || T > SB_DECODE_MAX_TOKENS || N < 1 || K < 32 || K % 32 != 0)
-    return fail(SB_E_INVALID_ARG, "sb_decode_linear: need 0<=T<=%d, N>=1, K%%32==0 (T=%d N=%d K=%d)",
+  if (T < 0 || T > SB_DECODE_MAX_TOKENS || N < 1 || N > (1 << 27) || K < 32 || K % 32 != 0)
+    return fail(SB_E_INVALID_ARG, "sb_decode_linear: need 0<=T<=%d, 1<=N<=2^27, K%%32==0 (T=%d N=%d K=%d)",
                 SB_DECODE_MAX_TOKENS, T, N, K);
   if (T == 0) return SB_OK;
   if (!x || !w || !out) return fail(SB_E_INVALID_ARG, "sb_decode_linear: null pointer");

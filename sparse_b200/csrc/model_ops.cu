@@ -643,7 +643,8 @@ int32_t sb_rope_append_mla(void *q, const void *k_pe, const void *kv, const int3
 }
 
 int32_t sb_argmax_rows(const void *logits, int32_t B, int32_t V, int64_t *out, void *stream) {
-  if (B < 0 || V < 1 || B > (1 << 24)) return fail(SB_E_INVALID_ARG, "sb_argmax_rows: bad shape (B=%d V=%d)", B, V);
+  if (B < 0 || V < 1 || B > (1 << 24) || V > (1 << 30))
+    return fail(SB_E_INVALID_ARG, "sb_argmax_rows: bad shape (B=%d V=%d)", B, V);
   if (B == 0) return SB_OK;
   if (!logits || !out) return fail(SB_E_INVALID_ARG, "sb_argmax_rows: null pointer");
   SB_CUDA_CHECK(launch_pdl(argmax_rows_kernel, dim3(B * kArgmaxCtas), dim3(kArgmaxThreads), 0,

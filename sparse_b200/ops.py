@@ -153,7 +153,7 @@ def _streams(rows: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
     if rows.dim() != 2 or weight.dim() != 2 or not 0 < rows.shape[0] <= _lib.DECODE_MAX_TOKENS:
         return False
     n, k = weight.shape
-    if n == 0 or k == 0 or k % 32 != 0 or rows.shape[1] != k or (bias is not None and bias.shape != (n,)):
+    if not 0 < n <= 2 ** 27 or k == 0 or k % 32 != 0 or rows.shape[1] != k or (bias is not None and bias.shape != (n,)):
         return False
     operands = [v for v in (rows, weight, bias) if v is not None]
     if any(v.dtype != torch.bfloat16 or not v.is_cuda or v.device != rows.device or not v.is_contiguous()

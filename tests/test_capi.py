@@ -83,6 +83,17 @@ def test_operands_off_their_load_width_are_refused():
         assert rc == -1 and b"aligned" in lib.sb_last_error_string()
 
 
+def test_sizes_beyond_the_index_arithmetic_are_refused():
+    from sparse_b200._lib import lib
+    ok = 1 << 20
+    for n in ((1 << 27) + 1, 1 << 29, (1 << 31) - 1):
+        assert lib.sb_decode_linear(ok, ok, None, 1, n, 32, ok, None) == -1
+        assert b"sb_decode_linear" in lib.sb_last_error_string()
+    for v in ((1 << 30) + 1, (1 << 31) - 1):
+        assert lib.sb_argmax_rows(ok, 1, v, ok, None) == -1
+        assert b"sb_argmax_rows" in lib.sb_last_error_string()
+
+
 def test_struct_layout_matches_header():
     from sparse_b200._lib import MoeLayer, lib
     assert C.sizeof(MoeLayer) == lib.sb_moe_layer_struct_bytes()
