@@ -155,3 +155,17 @@ def test_replaced_scratch_is_not_given_away_while_a_pass_uses_it():
     others = [torch.full((n,), 255, dtype=torch.uint8, device=DEV) for n in sizes for _ in range(4)]
     torch.cuda.synchronize()
     assert all(bool((o == 255).all()) for o in others)
+
+
+@pytest.mark.parametrize("name", ["TINY", "QWEN_MOE"])
+@pytest.mark.parametrize("t", [592, 593, 594, 599, 700, 887, 888, 889, 890, 895])
+def test_routing_beside_the_shared_pass_gives_the_bits_of_the_router_alone(name, t):
+    """The layer pass's own router tiles (six tokens, shared by two CTAs up to 888 tokens),
+    ragged last tiles among them."""
+    shape, w = getattr(synth, name), _weights(name)
+    runner = LayerRunner(w, shape.top_k, t)
+    x = _rows(t, shape.hidden, t)
+    _, *got = runner.forward(x)
+    want = ops.router_topk(x, w.router_w, shape.top_k, bias=w.router_bias, w_shared_gate=w.shared_gate_w)
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))

@@ -29,7 +29,8 @@ def test_expert_sort_at_its_size_limits(n, e):
 @pytest.mark.parametrize("h,e,k,dtype", [(2048, 60, 4, torch.bfloat16), (264, 256, 8, torch.bfloat16),
                                          (2048, 64, 6, torch.float32), (16384, 8, 2, torch.bfloat16)])
 def test_router_rows_do_not_depend_on_the_tile_shape(h, e, k, dtype):
-    """Every tile shape (tokens per CTA, CTAs per tile), ragged last tiles: the bits of one token alone."""
+    """Every tile shape of the router alone (tokens per CTA, CTAs per tile), ragged last tiles: the bits
+    of one token alone.  (The shapes beside a GEMM, from 593 tokens on: test_gpu_layer_calls.py.)"""
     torch.manual_seed(h + e)
     total = 1100
     x = torch.randn(total, h, device=DEV).to(dtype)
