@@ -526,8 +526,10 @@ int32_t launch_router_t(const void *x, const void *wg, const float *bias, const 
   if (T > slots && 4 * row <= room) launch = launch_router_tile<IN, 4, 4, 2>;
   if (T > 2 * slots && 7 * row <= room) launch = launch_router_tile<IN, 7, 4, 2>;
   if (T > 7 * slots / 2 && 7 * row <= room) launch = launch_router_tile<IN, 7, 4, 1>;
-  if (beside && T > 2 * slots && 6 * row <= room)
-    launch = T > 3 * slots ? launch_router_tile<IN, 6, 4, 1, 112> : launch_router_tile<IN, 6, 4, 2, 112>;
+  if constexpr (sizeof(IN) == 2) {       // (the layer pass, which asks for it, is bf16)
+    if (beside && T > 2 * slots && 6 * row <= room)
+      launch = T > 3 * slots ? launch_router_tile<IN, 6, 4, 1, 112> : launch_router_tile<IN, 6, 4, 2, 112>;
+  }
   return launch(x, wg, bias, wsg, T, H, E, K, renorm, fp32_logits, out_idx, out_w, out_logits, out_shared, stream);
 }
 
