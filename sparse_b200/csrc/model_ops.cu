@@ -293,9 +293,10 @@ int32_t launch_rope(__nv_bfloat16 *q, int q_stride, RopeSource k_rot, RopeSource
   const auto whole = [](const RopeSource &s) { return aligned(s.base, 16) && s.token % 8 == 0 && s.head % 8 == 0; };
   const bool vec = dk % 8 == 0 && dv % 8 == 0 && rope_dim % 16 == 0 && rope_dim <= 2 * kRopeTable && q_stride % 8 == 0 &&
                    aligned(q, 16) && whole(k_rot) && whole(k_rest) && whole(v) && aligned(cache_k, 16) && aligned(cache_v, 16);
-  // at most two waves' worth of CTAs: more would only repeat the angle table
+  // at most two waves of CTAs: more would only repeat the angle table
+  const int sms = sb_device_sm_count() > 0 ? sb_device_sm_count() : 148;
   const int items = (n_q * (rope_dim / 2) + n_kv * (dk - rope_dim / 2 + dv)) / (vec ? 8 : 1);
-  const int wanted = (items + kRopeThreads - 1) / kRopeThreads, room = (2 * 148 + T - 1) / T;
+  const int wanted = (items + kRopeThreads - 1) / kRopeThreads, room = (2 * sms + T - 1) / T;
   const dim3 grid(T, wanted < 1 ? 1 : wanted < room ? wanted : room);
   auto kern = vec ? rope_append_kernel<8> : rope_append_kernel<1>;
   SB_CUDA_CHECK(launch_pdl(kern, grid, dim3(kRopeThreads), 0, stream, q, q_stride, k_rot, k_rest, v, seq_of_token,
