@@ -230,8 +230,8 @@ int32_t sb_grouped_swiglu(const void *rows, const int32_t *tile_table,
  * a dense output buffer: rows of the local expert sort go straight to the rows
  * of a return buffer that a later sb_combine reads (see
  * sb_ep_exchange_dispatch_local).  Groups of any size (swept 16 rows at a time).
- * `T` is the caller's token count of this step (it selects the same K split,
- * hence the same summation order, as the step's other launches). */
+ * `T` is the caller's token count of this step, at least 1.  A row has the same
+ * bits as from the step's other launches: the summation order follows H and I. */
 int32_t sb_decode_experts_to(const void *x, const int32_t *item_of_slot, int32_t items_per_row,
                              const int32_t *tile_table, const int32_t *slot_of_expert, const void *w13,
                              const void *w2, const void *row_scale, int32_t H, int32_t I, int32_t n_slots,

@@ -100,7 +100,8 @@ class B200MoeBlock:
             return res
         if not self.use_graphs or not self._warm or x.shape[0] > self.runner.max_tokens:
             return self._pass(x, out)
-        self._drop_stale_graphs()
+        if self._graph_reserve != self.runner.reserves:
+            self._drop_stale_graphs()
         dst = self.runner.out[:x.shape[0]] if out is None else out
         key = (x.data_ptr(), x.shape[0], dst.data_ptr())
         if key not in self._graphs and len(self._graphs) >= 32:
@@ -132,12 +133,11 @@ class B200MoeBlock:
         return ent[3]
 
     def _drop_stale_graphs(self) -> None:
-        if self._graph_reserve != self.runner.reserves:
-            # A larger batch has replaced the runner's buffers, which the recorded passes write to.
-            torch.cuda.synchronize(self.device)
-            self._graphs.clear()
-            self._part_graphs.clear()
-            self._graph_reserve = self.runner.reserves
+        """A larger batch has replaced the runner's buffers, which the recorded passes write to."""
+        torch.cuda.synchronize(self.device)
+        self._graphs.clear()
+        self._part_graphs.clear()
+        self._graph_reserve = self.runner.reserves
 
     def forward_host(self, x_host: torch.Tensor, out_host: torch.Tensor) -> None:
         """x_host, out_host: pinned bf16 [T,H].  Copies in, runs the layer, copies
@@ -147,14 +147,14 @@ class B200MoeBlock:
             self._x_stage = torch.empty((max(t, self.runner.max_tokens), h), dtype=torch.bfloat16,
                                         device=self.device)
         xd = self._x_stage[:t]
-        stream = torch.cuda.current_stream(self.device)
-        parts = self._host_parts(x_host, out_host)
+        parts = self._host_parts(x_host, out_host) if t >= 3072 else 1
         if parts == 1:
             xd.copy_(x_host, non_blocking=True)
             out = self.forward_device(xd)
             out_host.copy_(out, non_blocking=True)
-            stream.synchronize()
+            torch.cuda.current_stream(self.device).synchronize()
             return
+        stream = torch.cuda.current_stream(self.device)
         # Part i + 1 comes in and part i - 1 goes out while part i is in the layer (a
         # row's result does not depend on the rows around it).
         graphs = self._graphs_of_parts(xd)
@@ -197,7 +197,8 @@ class B200MoeBlock:
         graphs of `forward_device`."""
         if not self.use_graphs:
             return None
-        self._drop_stale_graphs()
+        if self._graph_reserve != self.runner.reserves:
+            self._drop_stale_graphs()
         key = (xd.data_ptr(), xd.shape[0])
         if key in self._part_graphs:
             return self._part_graphs[key]
@@ -207,14 +208,14 @@ class B200MoeBlock:
         return None
 
     def _host_parts(self, x_host: torch.Tensor, out_host: torch.Tensor) -> int:
-        """Parts a host batch is passed in.  Splitting hides all copies but the first
-        part's in and the last part's out (75 ns a row each way), and costs the layer
-        time that two half batches take longer than one: from 3072 rows the copies
-        win (a batch below streams the expert weights twice for little).  A result that
-        is not row for row the input's counterpart, or that lies over other rows of
+        """Parts a host batch of at least 3072 rows is passed in.  Splitting hides all copies
+        but the first part's in and the last part's out (75 ns a row each way), and costs
+        the layer time that two half batches take longer than one: from 3072 rows the
+        copies win (a batch below streams the expert weights twice for little).  A result
+        that is not row for row the input's counterpart, or that lies over other rows of
         it, is copied as a whole."""
         tokens = x_host.shape[0]
-        if self._ep is not None or tokens < 3072 or tokens > self.runner.max_tokens:
+        if self._ep is not None or tokens > self.runner.max_tokens:
             return 1
         if out_host.shape != x_host.shape:
             return 1

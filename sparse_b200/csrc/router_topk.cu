@@ -503,9 +503,11 @@ int32_t launch_router_tile(const void *x, const void *wg, const float *bias, con
   return SB_OK;
 }
 
-// Tile shapes.  Up to seven tokens per CTA (28 running sums of two per lane are what 128
-// registers hold); fewer tokens per tile, and the router rows split over a cluster, while
-// that is what it takes to give every SM two CTAs (148 SMs):
+// Tile shapes.  Up to seven tokens per CTA: 28 running sums of two per lane, for which 128
+// registers are just too few (24 to 28 bytes a thread are spilled, 40 to 56 in the
+// six-token tiles of 112 registers, about 180 in fp32); fewer tokens per tile, and the
+// router rows split over a cluster, while that is what it takes to give every SM two CTAs
+// (148 SMs):
 //   T <= 74    1 token,  2 rows a pass, 4 CTAs per tile    T <= 592   4 tokens, 2 CTAs
 //   T <= 296   2 tokens, 4 rows a pass, 2 CTAs             T <= 1036  7 tokens, 2 CTAs
 //   above      7 tokens, 1 CTA
@@ -514,7 +516,9 @@ int32_t launch_router_tile(const void *x, const void *wg, const float *bias, con
 // warps of 96 registers are three on one scheduler, and that is what they leave two router
 // warps.  At 128 registers the router waits for the GEMM to end (4096 tokens 696 us per
 // layer against 680 us, 16384 tokens 2249 us against 2178 us); alone the wider tile is the
-// faster one (51 us against 59 us at 4096 tokens, 187 us against 207 us at 16384).
+// faster one (51 us against 59 us at 4096 tokens, 187 us against 207 us at 16384).  Up to 1024
+// tokens the shared pass holds 32 SMs and not all, and the layer's time is the same with
+// either tile (277 against 279 us at 1003 tokens, within the spread of its runs).
 template <typename IN>
 int32_t launch_router_t(const void *x, const void *wg, const float *bias, const void *wsg, int T,
                         int H, int E, int K, int renorm, int fp32_logits, int32_t *out_idx,

@@ -166,8 +166,7 @@ class LayerRunner:
             raise RuntimeError("rows %d..%d of a runner for %d" % (first_row, first_row + t, self.max_tokens))
         if t > self.max_tokens:
             self._reserve(t)
-        rows = slice(first_row, first_row + t)
-        dst = self.out[rows] if out is None else out
+        dst = self.out[first_row:first_row + t] if out is None else out
         L = MoeLayer()
         L.T, L.H, L.E, L.K, L.I, L.I_shared = t, w.hidden, w.num_experts, self.top_k, w.inter, w.shared_inter
         L.renorm, L.n_slots = int(self.renorm), w.n_slots
@@ -181,17 +180,20 @@ class LayerRunner:
         L.shared_w13 = w.shared_w13.data_ptr() if w.shared_w13 is not None else None
         L.shared_w2 = w.shared_w2.data_ptr() if w.shared_w2 is not None else None
         L.out = dst.data_ptr()
-        logits = self.logits[rows] if self.logits is not None else None
-        idx, weight = self.topk_idx[rows], self.topk_w[rows]
-        L.logits = logits.data_ptr() if logits is not None else None
-        L.topk_idx, L.topk_w = idx.data_ptr(), weight.data_ptr()
+        L.logits = None
+        if self.logits is not None:
+            L.logits = self.logits.data_ptr() + first_row * w.num_experts * (4 if self.fp32_logits else 2)
+        L.topk_idx = self.topk_idx.data_ptr() + first_row * self.top_k * 4
+        L.topk_w = self.topk_w.data_ptr() + first_row * self.top_k * 2
         L.ws, L.ws_bytes = self._ws_ptr, self._ws_bytes
         with torch.cuda.device(w.device):
             stream = torch.cuda.current_stream(w.device).cuda_stream
             check(lib.sb_moe_layer_forward(C.byref(L), self.status.data_ptr(), stream),
                   "sb_moe_layer_forward")
         self.last_launches = int(lib.sb_last_launch_count())
-        return dst, idx, weight, logits
+        # (the views behind the launch, not in front of it: 1 us each)
+        rows = slice(first_row, first_row + t)
+        return dst, self.topk_idx[rows], self.topk_w[rows], self.logits[rows] if self.logits is not None else None
 
     def check_status(self) -> None:
         """Host-synchronising check of the device status word (tests, debug)."""

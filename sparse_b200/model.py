@@ -14,7 +14,8 @@ initialised models of the two benchmark shapes:
   keys and values decompressed into the cache per head, vocabulary 102400.
 
 Per decode step every layer runs: RMSNorm (fused with the residual add) ->
-q/k/v projections (library GEMMs) -> rotary embedding + cache append ->
+q/k/v projections (the weight-streaming kernel up to 16 rows, library GEMMs
+above) -> rotary embedding + cache append ->
 decode attention over the cache -> output projection -> RMSNorm -> MoE block.
 All of it is stream-ordered with nothing read back, so the whole step (all
 layers, the lm_head GEMM and the argmax) is recorded once into a CUDA graph
@@ -155,8 +156,10 @@ class ShapedMoeModel:
             self.layers.append(ly)
         # enough key splits for about six CTAs per SM: a CTA streams its keys with
         # a few hundred bytes in flight per warp, so bandwidth comes from CTA count;
-        # but 64 keys a split at the longest, two turns of a CTA's 16 key groups: more
-        # splits of fewer keys only lengthen the merge
+        # but no more splits than leave each 64 keys, two turns of a CTA's 16 key groups,
+        # when the cache is full: more splits of fewer keys only lengthen the merge.  (The
+        # rule knows the cache's size, not how much of it is filled: a short context in a
+        # long cache keeps short splits.)
         sms = max(1, int(lib.sb_device_sm_count()) or 148)
         self.n_split = max(1, min(64, (6 * sms + batch * nh - 1) // (batch * nh), (max_seq + 63) // 64))
         ws = lib.sb_attn_decode_workspace_bytes(batch, nh, dv, self.n_split)
